@@ -56,6 +56,9 @@ enum : int { OVF_PAIRS = 1, OVF_MANIFOLDS = 2, OVF_EPA = 4, OVF_ISLAND = 8, OVF_
 // power of two above its contact count less one (9-16, 17-32, 33-64, 65-128, 129-256).  Each
 // bucket is a list of the body capacity.
 constexpr int SMALL_BUCKETS = 17, MID_BUCKETS = 5;
+// Contact islands above the per-warp tier: one CTA each, in two instances by footprint (contacts,
+// bodies); past the larger one's the whole grid solves them.
+constexpr int BLOCK_S_CONS = 2048, BLOCK_S_BODIES = 1024, BLOCK_L_CONS = 12288, BLOCK_L_BODIES = 6144;
 // The narrowphase takes the broadphase pairs grouped by the shapes' collide routine
 // (pair_class), so that the lanes of a warp run one routine.
 constexpr int PAIR_CLASSES = 8;
@@ -96,7 +99,7 @@ struct DevCounters {
     int mid_cursor_s;                 // cursor of the per-warp tier's small instance
     int pair_class[PAIR_CLASSES];     // broadphase pairs per collide class
     int pair_class_fill[PAIR_CLASSES];
-    int pad2[1];
+    int num_block_islands;            // contact islands of the larger per-CTA instance
 };
 
 // Settings copied into constant memory once per world.
@@ -505,7 +508,8 @@ struct DevWorld {
     cudaStream_t aux_stream;   // second stream: the per-CTA island solve runs beside the per-warp one
     cudaStream_t aux2_stream;  // third stream: the per-thread island solve beside both
     cudaStream_t aux3_stream;  // fourth stream: the per-warp solve of the islands past 32 contacts
-    cudaEvent_t ev_fork, ev_join, ev_join2, ev_join3;
+    cudaStream_t aux4_stream;  // fifth stream: the larger instance of the per-CTA solve
+    cudaEvent_t ev_fork, ev_join, ev_join2, ev_join3, ev_join4;
     int warp_blocks_per_sm;  // launch shape of the per-warp island solve
     int warp_carveout;       // shared-memory carveout (percent) of the per-warp island solve
     // persistent contact cache (double buffered by parity)
@@ -514,7 +518,9 @@ struct DevWorld {
     int *cache_parity;
     // island solve scratch
     int *root_flag;
-    int *small_list, *large_list;
+    int *small_list;
+    int *large_list;  // contact islands of the per-CTA tier: the smaller instance's from the front, the larger's from the back
+    float4 *solve_rows;  // 20 per contact: solver rows of the per-CTA tier in level order, one row per field
     int *scratch_order, *scratch_colour, *scratch_claim;
     int *contact_event;               // per manifold: 1 added, 2 persisted (listener.ts:58-79)
     unsigned long long *removed_keys;  // pairs in contact last step but not this step
@@ -549,7 +555,8 @@ struct DevWorld {
     int2 *hull_faces;                                  // first vertex index, vertex count
     int *hull_vidx;
     // giant islands (more constraints than giant_min): solved by the whole grid
-    int giant_min;
+    int giant_min;                         // islands with joints above this many constraints
+    int giant_min_contacts;                // islands of contacts above this many
     int giant_blocks;                      // blocks of the cooperative launch (co-resident)
     int *giant_list;
     unsigned long long *giant_claim;       // 4 x cap: contact claims, two parities | joint claims, two parities
@@ -897,6 +904,7 @@ void launch_update_bounds(DevWorld &w, cudaStream_t s);
 void upload_settings(const DevSettings &s, double spec64, cudaStream_t st);
 void launch_cache_begin(DevWorld &w, cudaStream_t s);
 size_t epa_scratch_bytes();
+int solve_rows_per_contact();
 size_t mesh_big_slot_bytes();
 constexpr int MESH_BIG_THREADS = 256;  // threads (and 32-manifold slots) of the mesh pairs' big-pool pass
 void upload_settings_adjoint(const DevSettings &s, cudaStream_t st);

@@ -553,7 +553,7 @@ __device__ __forceinline__ int bucketed_island(const int *list, size_t cap, cons
 }
 
 // Island classes of k_island_classify: a per-thread or per-warp size bucket, or one of these.
-enum : int { CL_NONE = -1, CL_MID0 = 100, CL_GIANT = 1000, CL_SMALL_JOINT, CL_LARGE_JOINT, CL_LARGE };
+enum : int { CL_NONE = -1, CL_MID0 = 100, CL_GIANT = 1000, CL_SMALL_JOINT, CL_LARGE_JOINT, CL_LARGE, CL_BLOCK };
 
 __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) {
     const int ni = w.ctr->num_islands;
@@ -568,7 +568,8 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
             const int nc = w.island_cons_count[i], nb = w.island_body_count[i];
             const int nj = joint_total(w) > 0 ? w.island_joint_count[i] : 0;
             tot = nc + nj;
-            if (nc + nj > w.giant_min) {  // a pile: the whole grid solves it
+            if (nj > 0 ? nc + nj > w.giant_min : nc > w.giant_min_contacts || nb > BLOCK_L_BODIES) {
+                // a pile: the whole grid solves it
                 cls = CL_GIANT;
             } else if (nj > 0) {
                 // islands with joints: one thread in the reference's exact order when small (a lone
@@ -585,7 +586,7 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
                 if (b < 2 && nb > WARP_S_BODIES) b = 2;
                 cls = CL_MID0 + b;
             } else {
-                cls = CL_LARGE;
+                cls = nc <= BLOCK_S_CONS && nb <= BLOCK_S_BODIES ? CL_LARGE : CL_BLOCK;
             }
         }
         const int mx = __reduce_max_sync(FULL, tot);
@@ -605,6 +606,9 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
         } else if (cls == CL_LARGE) {
             ctr = &w.ctr->num_large_islands;
             list = large_list;
+        } else if (cls == CL_BLOCK) {  // from the back of the same list
+            ctr = &w.ctr->num_block_islands;
+            list = large_list;
         } else if (cls >= CL_MID0) {
             ctr = &w.ctr->mid_bucket[cls - CL_MID0];
             list = w.mid_list + (size_t)(cls - CL_MID0) * w.cap;
@@ -620,7 +624,8 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
             if (total) atomicAdd(total, cnt);
         }
         slot = __shfl_sync(same, slot, leader);
-        if (ctr) list[slot + __popc(same & ((1u << lane) - 1u))] = i;
+        slot += __popc(same & ((1u << lane) - 1u));
+        if (ctr) list[cls == CL_BLOCK ? w.cap - 1 - slot : slot] = i;
     }
 }
 
@@ -690,52 +695,59 @@ __device__ __forceinline__ void apply_impulse(BodyRef &A, BodyRef &B, float imA,
     }
 }
 
-// warm start of one constraint (contact-constraints.ts:906-955)
-__device__ void warm_start_con(ContactConstraint &c, BodyRef &A, BodyRef &B, float ratio) {
-    for (int k = 0; k < c.n; k++) {
-        ContactPoint &p = c.p[k];
-        if (p.eff_t1 != 0.f || p.eff_t2 != 0.f) {
-            p.lam_t1 *= ratio;
-            apply_impulse(A, B, c.invMassA, c.invMassB, c.t1, p.rA, p.rB, p.lam_t1);
-            p.lam_t2 *= ratio;
-            apply_impulse(A, B, c.invMassA, c.invMassB, c.t2, p.rA, p.rB, p.lam_t2);
+// The rows of one contact point, P: a ContactPoint or a register copy of its solver fields.
+// warm start of one point (contact-constraints.ts:906-955)
+template <class P>
+__device__ __forceinline__ void warm_start_point(P &p, BodyRef &A, BodyRef &B, float imA, float imB, float3 n, float3 t1,
+                                                 float3 t2, float ratio) {
+    if (p.eff_t1 != 0.f || p.eff_t2 != 0.f) {
+        p.lam_t1 *= ratio;
+        apply_impulse(A, B, imA, imB, t1, p.rA, p.rB, p.lam_t1);
+        p.lam_t2 *= ratio;
+        apply_impulse(A, B, imA, imB, t2, p.rA, p.rB, p.lam_t2);
+    }
+    p.lam_n *= ratio;
+    apply_impulse(A, B, imA, imB, n, p.rA, p.rB, p.lam_n);
+}
+// one PGS pass over one contact (contact-constraints.ts:963-1053): the friction rows of every
+// point, then the normal rows
+template <class P>
+__device__ __forceinline__ void friction_point(P &p, BodyRef &A, BodyRef &B, float imA, float imB, float3 t1, float3 t2,
+                                               float friction) {
+    if (p.eff_t1 != 0.f || p.eff_t2 != 0.f) {
+        float l1 = total_lambda(A, B, t1, p.rA, p.rB, p.eff_t1, p.lam_t1, 0.f);
+        float l2 = total_lambda(A, B, t2, p.rA, p.rB, p.eff_t2, p.lam_t2, 0.f);
+        float mf = friction * p.lam_n;
+        float fm = l1 * l1 + l2 * l2;
+        if (fm > mf * mf) {
+            float s = mf / sqrtf(fm);
+            l1 *= s;
+            l2 *= s;
         }
-        p.lam_n *= ratio;
-        apply_impulse(A, B, c.invMassA, c.invMassB, c.normal, p.rA, p.rB, p.lam_n);
+        float d1 = l1 - p.lam_t1;
+        p.lam_t1 = l1;
+        apply_impulse(A, B, imA, imB, t1, p.rA, p.rB, d1);
+        float d2 = l2 - p.lam_t2;
+        p.lam_t2 = l2;
+        apply_impulse(A, B, imA, imB, t2, p.rA, p.rB, d2);
     }
 }
-
-// one PGS pass over one contact (contact-constraints.ts:963-1053)
+template <class P>
+__device__ __forceinline__ void normal_point(P &p, BodyRef &A, BodyRef &B, float imA, float imB, float3 n) {
+    float tl = total_lambda(A, B, n, p.rA, p.rB, p.eff_n, p.lam_n, p.bias_n);
+    tl = fmaxf(0.f, tl);
+    float dl = tl - p.lam_n;
+    p.lam_n = tl;
+    apply_impulse(A, B, imA, imB, n, p.rA, p.rB, dl);
+}
+__device__ void warm_start_con(ContactConstraint &c, BodyRef &A, BodyRef &B, float ratio) {
+    for (int k = 0; k < c.n; k++)
+        warm_start_point(c.p[k], A, B, c.invMassA, c.invMassB, c.normal, c.t1, c.t2, ratio);
+}
 __device__ void solve_velocity_con(ContactConstraint &c, BodyRef &A, BodyRef &B) {
     if (A.motion != DYNAMIC && B.motion != DYNAMIC) return;
-    for (int k = 0; k < c.n; k++) {
-        ContactPoint &p = c.p[k];
-        if (p.eff_t1 != 0.f || p.eff_t2 != 0.f) {
-            float l1 = total_lambda(A, B, c.t1, p.rA, p.rB, p.eff_t1, p.lam_t1, 0.f);
-            float l2 = total_lambda(A, B, c.t2, p.rA, p.rB, p.eff_t2, p.lam_t2, 0.f);
-            float mf = c.friction * p.lam_n;
-            float fm = l1 * l1 + l2 * l2;
-            if (fm > mf * mf) {
-                float s = mf / sqrtf(fm);
-                l1 *= s;
-                l2 *= s;
-            }
-            float d1 = l1 - p.lam_t1;
-            p.lam_t1 = l1;
-            apply_impulse(A, B, c.invMassA, c.invMassB, c.t1, p.rA, p.rB, d1);
-            float d2 = l2 - p.lam_t2;
-            p.lam_t2 = l2;
-            apply_impulse(A, B, c.invMassA, c.invMassB, c.t2, p.rA, p.rB, d2);
-        }
-    }
-    for (int k = 0; k < c.n; k++) {
-        ContactPoint &p = c.p[k];
-        float tl = total_lambda(A, B, c.normal, p.rA, p.rB, p.eff_n, p.lam_n, p.bias_n);
-        tl = fmaxf(0.f, tl);
-        float dl = tl - p.lam_n;
-        p.lam_n = tl;
-        apply_impulse(A, B, c.invMassA, c.invMassB, c.normal, p.rA, p.rB, dl);
-    }
+    for (int k = 0; k < c.n; k++) friction_point(c.p[k], A, B, c.invMassA, c.invMassB, c.t1, c.t2, c.friction);
+    for (int k = 0; k < c.n; k++) normal_point(c.p[k], A, B, c.invMassA, c.invMassB, c.normal);
 }
 
 // rotation step (rigid-body-step.ts:55-97)
@@ -756,7 +768,46 @@ struct PoseRef {
     float4 q;
 };
 
-// position solve of one contact (contact-constraints.ts:1098-1216); returns true if an impulse was applied
+// one side of a contact in the position solve: the body's motion, degrees of freedom and local inertia
+struct PoseSide {
+    int motion, dof;
+    float4 inertia_rot;
+    float3 inv_inertia;
+    float im;
+};
+// position solve of one contact point (contact-constraints.ts:1098-1216) with the contact's
+// rotations and inverse inertias; returns true if an impulse was applied
+__device__ __forceinline__ bool position_point(float3 localA, float3 localB, float3 normal, PoseRef &PA, PoseRef &PB,
+                                               const Mat3 &RA, const Mat3 &RB, const Sym3 &IA, const Sym3 &IB,
+                                               const PoseSide &SA, const PoseSide &SB) {
+    float3 pa = PA.com + mmul(RA, localA);
+    float3 pb = PB.com + mmul(RB, localB);
+    float sep = dot3(pb - pa, normal) + c_settings.slop;
+    sep = fmaxf(sep, -c_settings.max_pen);
+    if (sep >= 0.f) return false;
+    float3 mid = (pa + pb) * 0.5f;
+    float3 rA = mid - PA.com, rB = mid - PB.com;
+    float iem = inv_eff_mass(SA.motion == DYNAMIC, SB.motion == DYNAMIC, SA.im, SB.im, IA, IB, rA, rB, normal);
+    if (iem == 0.f) return false;
+    float eff = 1.f / iem;
+    float lambda = -eff * c_settings.baumgarte * sep;
+    if (SA.motion == DYNAMIC) {
+        PA.com = PA.com - normal * (lambda * SA.im);
+        if (!(SA.dof & 1)) PA.com.x = 0.f;
+        if (!(SA.dof & 2)) PA.com.y = 0.f;
+        if (!(SA.dof & 4)) PA.com.z = 0.f;
+        PA.q = rotation_step(PA.q, -(symmul(IA, cross3(rA, normal)) * lambda));
+    }
+    if (SB.motion == DYNAMIC) {
+        PB.com = PB.com + normal * (lambda * SB.im);
+        if (!(SB.dof & 1)) PB.com.x = 0.f;
+        if (!(SB.dof & 2)) PB.com.y = 0.f;
+        if (!(SB.dof & 4)) PB.com.z = 0.f;
+        PB.q = rotation_step(PB.q, symmul(IB, cross3(rB, normal)) * lambda);
+    }
+    return true;
+}
+// position solve of one contact; returns true if an impulse was applied
 __device__ bool solve_position_con(DevWorld &w, const ContactConstraint &c, PoseRef &PA, PoseRef &PB, int ma, int mb,
                                    uint32_t fa, uint32_t fb) {
     if (ma != DYNAMIC && mb != DYNAMIC) return false;
@@ -764,39 +815,11 @@ __device__ bool solve_position_con(DevWorld &w, const ContactConstraint &c, Pose
     // rotations and inverse inertias are taken once per contact, as the reference does
     const Mat3 RA = quat_to_mat(PA.q), RB = quat_to_mat(PB.q);
     Sym3 IA{0, 0, 0, 0, 0, 0}, IB{0, 0, 0, 0, 0, 0};
-    if (ma == DYNAMIC) IA = world_inv_inertia(PA.q, w.inertia_rot[c.a], xyz(w.inv_inertia[c.a]), dof_of(fa));
-    if (mb == DYNAMIC) IB = world_inv_inertia(PB.q, w.inertia_rot[c.b], xyz(w.inv_inertia[c.b]), dof_of(fb));
-    for (int k = 0; k < c.n; k++) {
-        const ContactPoint &p = c.p[k];
-        float3 pa = PA.com + mmul(RA, p.localA);
-        float3 pb = PB.com + mmul(RB, p.localB);
-        float sep = dot3(pb - pa, c.normal) + c_settings.slop;
-        sep = fmaxf(sep, -c_settings.max_pen);
-        if (sep >= 0.f) continue;
-        float3 mid = (pa + pb) * 0.5f;
-        float3 rA = mid - PA.com, rB = mid - PB.com;
-        float iem = inv_eff_mass(ma == DYNAMIC, mb == DYNAMIC, c.invMassA, c.invMassB, IA, IB, rA, rB, c.normal);
-        if (iem == 0.f) continue;
-        float eff = 1.f / iem;
-        float lambda = -eff * c_settings.baumgarte * sep;
-        if (ma == DYNAMIC) {
-            PA.com = PA.com - c.normal * (lambda * c.invMassA);
-            int d = dof_of(fa);
-            if (!(d & 1)) PA.com.x = 0.f;
-            if (!(d & 2)) PA.com.y = 0.f;
-            if (!(d & 4)) PA.com.z = 0.f;
-            PA.q = rotation_step(PA.q, -(symmul(IA, cross3(rA, c.normal)) * lambda));
-        }
-        if (mb == DYNAMIC) {
-            PB.com = PB.com + c.normal * (lambda * c.invMassB);
-            int d = dof_of(fb);
-            if (!(d & 1)) PB.com.x = 0.f;
-            if (!(d & 2)) PB.com.y = 0.f;
-            if (!(d & 4)) PB.com.z = 0.f;
-            PB.q = rotation_step(PB.q, symmul(IB, cross3(rB, c.normal)) * lambda);
-        }
-        any = true;
-    }
+    PoseSide SA{ma, dof_of(fa), {}, {}, c.invMassA}, SB{mb, dof_of(fb), {}, {}, c.invMassB};
+    if (ma == DYNAMIC) IA = world_inv_inertia(PA.q, w.inertia_rot[c.a], xyz(w.inv_inertia[c.a]), SA.dof);
+    if (mb == DYNAMIC) IB = world_inv_inertia(PB.q, w.inertia_rot[c.b], xyz(w.inv_inertia[c.b]), SB.dof);
+    for (int k = 0; k < c.n; k++)
+        any = position_point(c.p[k].localA, c.p[k].localB, c.normal, PA, PB, RA, RB, IA, IB, SA, SB) || any;
     return any;
 }
 
@@ -1068,14 +1091,15 @@ __global__ void __launch_bounds__(128) k_solve_small(DevWorld w, CacheTables ct,
     }
 }
 
+#include "cc_solve_block.cuh"
+
 // ---------------------------------------------------------------------------
-// large islands: one CTA per island, contacts sorted by the reference key,
+// large islands with joints: one CTA per island, contacts sorted by the reference key,
 // greedily coloured in that order and swept colour by colour
 // ---------------------------------------------------------------------------
 constexpr int LARGE_BLOCK = 256;
 constexpr int JOINT_COLOURS = 64;  // joint colours of the per-CTA solve; the rest go to one thread
 
-template <bool JOINTS>
 __global__ void __launch_bounds__(LARGE_BLOCK) k_solve_large(DevWorld w, CacheTables ct, const int *large_list,
                                                               int *scratch_order, int *scratch_colour,
                                                               int *scratch_claim, float dt, float ratio,
@@ -1085,7 +1109,7 @@ __global__ void __launch_bounds__(LARGE_BLOCK) k_solve_large(DevWorld w, CacheTa
     __shared__ int s_ncol;
     __shared__ int s_colour_start[257];
     __shared__ int s_jstart[JOINT_COLOURS + 2];
-    int nl = JOINTS ? w.ctr->num_large_joint_islands : w.ctr->num_large_islands;
+    int nl = w.ctr->num_large_joint_islands;
     CacheRecord *crecs = ct.recs[*ct.parity];
     for (int li = blockIdx.x; li < nl; li += gridDim.x) {
         int isl = large_list[li];
@@ -1111,7 +1135,7 @@ __global__ void __launch_bounds__(LARGE_BLOCK) k_solve_large(DevWorld w, CacheTa
             for (int k = threadIdx.x; k < nb; k += blockDim.x) prepare_body(w, bl[k]);
         // the island's joints in index order (warm start) and in (priority, index) order
         // (sortConstraintIds constraints.ts:248-261)
-        int nj = JOINTS ? w.island_joint_count[isl] : 0;
+        int nj = w.island_joint_count[isl];
         const int *jl = w.island_joints + (nj > 0 ? w.island_joint_off[isl] : 0);
         int *j_idx = const_cast<int *>(jl) + w.max_joints;
         int *j_pri = j_idx + w.max_joints;
@@ -1986,6 +2010,7 @@ __global__ void __launch_bounds__(GIANT_BLOCK) k_solve_giant(DevWorld w, CacheTa
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+int solve_rows_per_contact() { return SOLVE_ROWS; }
 static CacheTables tables_of(DevWorld &w) {
     CacheTables ct;
     ct.keys[0] = w.cache_keys[0];
@@ -2108,10 +2133,29 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
     // the per-CTA and per-warp classes hold disjoint islands: run them side by side
     cudaEventRecord(w.ev_fork, s);
     cudaStreamWaitEvent(w.aux_stream, w.ev_fork, 0);
-    k_solve_large<false><<<device_sm_count() * 2, LARGE_BLOCK, 0, w.aux_stream>>>(
-        w, ct, w.large_list, w.scratch_order, w.scratch_colour, w.scratch_claim, dt, ratio, phase);
+    static bool block_attr_set = false;
+    if (!block_attr_set) {
+        cudaFuncSetAttribute(k_solve_block<BlockTierS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)BlockTierS::SMEM);
+        cudaFuncSetAttribute(k_solve_block<BlockTierL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)BlockTierL::SMEM);
+        block_attr_set = true;
+    }
+    // no more blocks than the world can have islands of the instance's size; none at all where it
+    // cannot have one
+    const int sms = device_sm_count();
+    const int max_s = w.max_manifolds / WARP_MAX_CONS + w.n / WARP_MAX_BODIES + 1;
+    const int max_l = w.max_manifolds / BLOCK_S_CONS + w.n / BLOCK_S_BODIES;
+    k_solve_block<BlockTierS><<<max_s < 2 * sms ? max_s : 2 * sms, BlockTierS::THREADS, BlockTierS::SMEM,
+                                w.aux_stream>>>(w, ct, w.large_list, 1, &w.ctr->num_large_islands, dt, ratio, phase);
+    if (max_l > 0) {
+        cudaStreamWaitEvent(w.aux4_stream, w.ev_fork, 0);
+        k_solve_block<BlockTierL><<<max_l < sms ? max_l : sms, BlockTierL::THREADS, BlockTierL::SMEM, w.aux4_stream>>>(
+            w, ct, w.large_list + w.cap - 1, -1, &w.ctr->num_block_islands, dt, ratio, phase);
+        cudaEventRecord(w.ev_join4, w.aux4_stream);
+    }
     if (joints)
-        k_solve_large<true><<<device_sm_count() * 2, LARGE_BLOCK, 0, w.aux_stream>>>(
+        k_solve_large<<<device_sm_count() * 2, LARGE_BLOCK, 0, w.aux_stream>>>(
             w, ct, w.large_joint_list, w.scratch_order, w.scratch_colour, w.scratch_claim, dt, ratio, phase);
     cudaEventRecord(w.ev_join, w.aux_stream);
     // the per-warp tier's large instance on a fourth stream, its small instance on the step's
@@ -2123,9 +2167,14 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
         w, ct, dt, ratio, phase, 0, 2, &w.ctr->mid_cursor_s);
     cudaStreamWaitEvent(s, w.ev_join, 0);
     cudaStreamWaitEvent(s, w.ev_join3, 0);
+    if (max_l > 0) cudaStreamWaitEvent(s, w.ev_join4, 0);
     if (!split) cudaStreamWaitEvent(s, w.ev_join2, 0);
     // giant islands: a cooperative launch (all blocks co-resident), after the other tiers so that
-    // it runs alone; it returns at once when the step has no giant island
+    // it runs alone; it returns at once when the step has no giant island, and is left out (9 us)
+    // where the world is too small for one
+    const int nj = w.num_hinges + w.num_swings + w.num_others + w.num_sixdofs;
+    const bool giant_possible = w.max_manifolds > w.giant_min_contacts || w.n > BLOCK_L_BODIES ||
+                                (nj > 0 && w.max_manifolds + nj > w.giant_min);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)w.giant_blocks);
     cfg.blockDim = dim3(GIANT_BLOCK);
@@ -2135,7 +2184,7 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (w.giant_blocks > 0) cudaLaunchKernelEx(&cfg, k_solve_giant, w, ct, dt, ratio, phase);
+    if (w.giant_blocks > 0 && giant_possible) cudaLaunchKernelEx(&cfg, k_solve_giant, w, ct, dt, ratio, phase);
 }
 
 // ---------------------------------------------------------------------------

@@ -125,6 +125,16 @@ static void drop_graph(cc_world *W) {
     }
 }
 
+// Islands with joints go to the whole grid above the given number of constraints.  So do islands of
+// contacts when the threshold is set; at its default the per-CTA tier keeps them up to its capacity
+// (a 16 x 16 x 16 heap of 11,776 contacts: 1.9 ms on one CTA, 17.5 ms on the grid, whose every
+// colour costs two grid-wide memory round trips).
+constexpr int GIANT_MIN_DEFAULT = 8192;
+static void set_giant_min(DevWorld &w, int v) {
+    w.giant_min = v;
+    w.giant_min_contacts = v == GIANT_MIN_DEFAULT || v > BLOCK_L_CONS ? BLOCK_L_CONS : v;
+}
+
 // continuous-collision buffers, made when the first LINEAR_CAST body arrives
 static int ensure_ccd_buffers(cc_world *W) {
     DevWorld &w = W->w;
@@ -492,6 +502,12 @@ int cc_world_create(const cc_world_settings *s, cc_world **out) {
     ALLOC(root_flag, cap);
     ALLOC(small_list, (size_t)cap * SMALL_BUCKETS);
     ALLOC(large_list, cap);
+    // written before it is read in every step: not cleared
+    if ((r = cuda_ok(cudaMalloc((void **)&w.solve_rows, sizeof(float4) * (size_t)solve_rows_per_contact() *
+                                                            (size_t)w.max_manifolds))) != CC_OK) {
+        cc_world_destroy(W);
+        return r;
+    }
     ALLOC(scratch_order, w.max_manifolds);
     ALLOC(scratch_colour, w.max_manifolds);
     ALLOC(scratch_claim, (size_t)cap + (size_t)w.max_manifolds + 16);
@@ -504,22 +520,24 @@ int cc_world_create(const cc_world_settings *s, cc_world **out) {
     ALLOC(giant_count, 4 * (GIANT_COLOURS + 2));
 #undef ALLOC
     // islands with more constraints than this are solved by the whole grid (launch-shape tunable)
-    w.giant_min = 8192;
+    set_giant_min(w, GIANT_MIN_DEFAULT);
     if (const char *e = getenv("CRASHCAT_GIANT_MIN")) {
         int v = atoi(e);
-        if (v >= 1) w.giant_min = v;
+        if (v >= 1) set_giant_min(w, v);
     }
     w.giant_blocks = giant_blocks_for_device();
     if (const char *e = getenv("CRASHCAT_GIANT_BLOCKS")) {  // launch-shape tunable, at most one per SM
         int v = atoi(e);
         if (v >= 1 && v < w.giant_blocks) w.giant_blocks = v;
     }
-    if (w.giant_blocks <= 0) w.giant_min = 0x7fffffff;
+    if (w.giant_blocks <= 0) set_giant_min(w, 0x7fffffff);
     if ((r = cuda_ok(cudaStreamCreateWithFlags(&W->stream, cudaStreamNonBlocking))) != CC_OK ||
         (r = cuda_ok(cudaStreamCreateWithFlags(&w.aux_stream, cudaStreamNonBlocking))) != CC_OK ||
         (r = cuda_ok(cudaStreamCreateWithFlags(&w.aux2_stream, cudaStreamNonBlocking))) != CC_OK ||
         (r = cuda_ok(cudaStreamCreateWithFlags(&w.aux3_stream, cudaStreamNonBlocking))) != CC_OK ||
+        (r = cuda_ok(cudaStreamCreateWithFlags(&w.aux4_stream, cudaStreamNonBlocking))) != CC_OK ||
         (r = cuda_ok(cudaEventCreateWithFlags(&w.ev_join3, cudaEventDisableTiming))) != CC_OK ||
+        (r = cuda_ok(cudaEventCreateWithFlags(&w.ev_join4, cudaEventDisableTiming))) != CC_OK ||
         (r = cuda_ok(cudaEventCreateWithFlags(&w.ev_fork, cudaEventDisableTiming))) != CC_OK ||
         (r = cuda_ok(cudaEventCreateWithFlags(&w.ev_join, cudaEventDisableTiming))) != CC_OK ||
         (r = cuda_ok(cudaEventCreateWithFlags(&w.ev_join2, cudaEventDisableTiming))) != CC_OK) {
@@ -553,7 +571,7 @@ int cc_world_destroy(cc_world *W) {
                     w.island_cons_count, w.island_body_off, w.island_cons_off, w.island_bodies, w.island_cons,
                     w.island_fill_b, w.island_fill_c, w.iter_ovr, w.island_iters, w.inv_inertia_world, w.scan_tmp, w.ctr, w.scene,
                     w.node_world, w.epa_items, w.epa_packed, w.epa_scratch, w.epa_fallback, w.cache_keys[0], w.cache_keys[1], w.cache_recs[0],
-                    w.cache_recs[1], w.cache_parity, w.root_flag, w.small_list, w.large_list, w.scratch_order,
+                    w.cache_recs[1], w.cache_parity, w.root_flag, w.small_list, w.large_list, w.solve_rows, w.scratch_order,
                     w.scratch_colour, w.scratch_claim, w.mid_list, w.body_local, w.contact_event,
                     w.removed_keys, W->d_state_rows, w.hinges, w.island_joints, w.island_joint_count,
                     w.island_joint_off, w.island_fill_j, w.joint_wake, w.joint_partners, w.swings, w.others, w.sixdofs, w.frames,
@@ -583,6 +601,8 @@ int cc_world_destroy(cc_world *W) {
     if (w.aux_stream) cudaStreamDestroy(w.aux_stream);
     if (w.aux2_stream) cudaStreamDestroy(w.aux2_stream);
     if (w.aux3_stream) cudaStreamDestroy(w.aux3_stream);
+    if (w.aux4_stream) cudaStreamDestroy(w.aux4_stream);
+    if (w.ev_join4) cudaEventDestroy(w.ev_join4);
     if (w.ev_join3) cudaEventDestroy(w.ev_join3);
     if (w.ev_fork) cudaEventDestroy(w.ev_fork);
     if (w.ev_join) cudaEventDestroy(w.ev_join);
@@ -2016,7 +2036,7 @@ static int tune_apply(cc_world *W, const TuneShape &t) {
     w.epa_fetch_warp = t.epa_lockstep;
     w.warp_blocks_per_sm = t.warp_blocks_per_sm;
     W->dev_settings.small_island_max_cons = t.small_max;
-    w.giant_min = t.giant_min;
+    set_giant_min(w, t.giant_min);
     drop_graph(W);
     return CC_OK;
 }
