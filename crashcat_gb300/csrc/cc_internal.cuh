@@ -58,7 +58,8 @@ enum : int { OVF_PAIRS = 1, OVF_MANIFOLDS = 2, OVF_EPA = 4, OVF_ISLAND = 8, OVF_
 constexpr int SMALL_BUCKETS = 17, MID_BUCKETS = 5;
 // Contact islands above the per-warp tier: one CTA each, in two instances by footprint (contacts,
 // bodies); past the larger one's the whole grid solves them.
-constexpr int BLOCK_S_CONS = 2048, BLOCK_S_BODIES = 1024, BLOCK_L_CONS = 12288, BLOCK_L_BODIES = 6144;
+constexpr int BLOCK_S_CONS = 4096, BLOCK_S_BODIES = 2048, BLOCK_L_CONS = 12288, BLOCK_L_BODIES = 6144;
+constexpr int SOLVE_SWEEPS = 12;  // sweeps of one schedule of the per-CTA tier (a warm start and ten iterations fit)
 // The narrowphase takes the broadphase pairs grouped by the shapes' collide routine
 // (pair_class), so that the lanes of a warp run one routine.
 constexpr int PAIR_CLASSES = 8;
@@ -520,7 +521,9 @@ struct DevWorld {
     int *root_flag;
     int *small_list;
     int *large_list;  // contact islands of the per-CTA tier: the smaller instance's from the front, the larger's from the back
-    float4 *solve_rows;  // 20 per contact: solver rows of the per-CTA tier in level order, one row per field
+    float4 *solve_rows;  // 20 per contact: solver rows of the per-CTA tier, one row per field
+    uint16_t *solve_tasks;   // SOLVE_SWEEPS per contact: the tier's visits in level order
+    uint32_t *solve_chunks;  // SOLVE_SWEEPS per contact: the visits in chunks of at most 32
     int *scratch_order, *scratch_colour, *scratch_claim;
     int *contact_event;               // per manifold: 1 added, 2 persisted (listener.ts:58-79)
     unsigned long long *removed_keys;  // pairs in contact last step but not this step

@@ -504,7 +504,11 @@ int cc_world_create(const cc_world_settings *s, cc_world **out) {
     ALLOC(large_list, cap);
     // written before it is read in every step: not cleared
     if ((r = cuda_ok(cudaMalloc((void **)&w.solve_rows, sizeof(float4) * (size_t)solve_rows_per_contact() *
-                                                            (size_t)w.max_manifolds))) != CC_OK) {
+                                                            (size_t)w.max_manifolds))) != CC_OK ||
+        (r = cuda_ok(cudaMalloc((void **)&w.solve_tasks, sizeof(uint16_t) * SOLVE_SWEEPS * (size_t)w.max_manifolds))) !=
+            CC_OK ||
+        (r = cuda_ok(cudaMalloc((void **)&w.solve_chunks, sizeof(uint32_t) * SOLVE_SWEEPS *
+                                                              (size_t)w.max_manifolds))) != CC_OK) {
         cc_world_destroy(W);
         return r;
     }
@@ -571,7 +575,7 @@ int cc_world_destroy(cc_world *W) {
                     w.island_cons_count, w.island_body_off, w.island_cons_off, w.island_bodies, w.island_cons,
                     w.island_fill_b, w.island_fill_c, w.iter_ovr, w.island_iters, w.inv_inertia_world, w.scan_tmp, w.ctr, w.scene,
                     w.node_world, w.epa_items, w.epa_packed, w.epa_scratch, w.epa_fallback, w.cache_keys[0], w.cache_keys[1], w.cache_recs[0],
-                    w.cache_recs[1], w.cache_parity, w.root_flag, w.small_list, w.large_list, w.solve_rows, w.scratch_order,
+                    w.cache_recs[1], w.cache_parity, w.root_flag, w.small_list, w.large_list, w.solve_rows, w.solve_tasks, w.solve_chunks, w.scratch_order,
                     w.scratch_colour, w.scratch_claim, w.mid_list, w.body_local, w.contact_event,
                     w.removed_keys, W->d_state_rows, w.hinges, w.island_joints, w.island_joint_count,
                     w.island_joint_off, w.island_fill_j, w.joint_wake, w.joint_partners, w.swings, w.others, w.sixdofs, w.frames,
