@@ -2301,51 +2301,159 @@ __global__ void k_ccd_scatter(DevWorld w) {
     }
 }
 
-// sortCCDBodies update.ts:1583-1611 and resolveCCDContacts update.ts:1616-1670, one thread per
+// one record's move: the displacement times `move` (1 without a hit)
+__device__ void ccd_move(DevWorld &w, const CcdRec &c, float move) {
+    const int a = c.body;
+    const uint32_t fa = w.flags[a];
+    const float3 p = xyz(w.pos[a]) + xyz(c.delta) * move;
+    const float3 cm = p + qrot(w.quat[a], shape_com(w, a, fa, w.shape[a]));
+    w.pos[a] = make_float4(p.x, p.y, p.z, 0.f);
+    w.com[a] = make_float4(cm.x, cm.y, cm.z, 0.f);
+}
+// one hit record's turn: the cascade (cb: the record in the slot of the body it hits, null when
+// that body has none), applyCCD, the move, the wake of the body hit
+__device__ void ccd_hit(DevWorld &w, CcdRec &c, CcdRec *cb, float2 &lam) {
+    const int b = c.hit;
+    if (cb && cb->hit >= 0 && cb->point.w > c.point.w) {
+        cb->hit = -1;
+        cb->fps = c.point.w;
+    }
+    ccd_apply(w, c, c.body, b, lam);
+    const float move = c.fps;
+    if (sleeping_of(w.flags[b])) {
+        w.flags[b] &= ~F_SLEEPING;
+        reset_sleep(w, b);
+    }
+    ccd_move(w, c, move);
+}
+
+// sortCCDBodies update.ts:1583-1611 and resolveCCDContacts update.ts:1616-1670, one CTA per
 // world.  A body's record index names its slot in creation (body index) order; after the sort
-// the cascade reads the record that now sits in that slot, as the reference does.
-__global__ void k_ccd_resolve(DevWorld w) {
-    if (w.ctr->num_ccd == 0) return;
+// the cascade reads the record that now sits in that slot, as the reference does.  The sort and
+// the moves without a hit take all threads (one thread on two heap sorts and 1,194 moves from
+// global memory took 4.8 ms); the hits, a few in a hundred, follow one another on one thread.  A move
+// without a hit is seen by others only as the body that a later record hits, so it may wait
+// until such a record needs it, or until the end.  Worlds of more than CCD_SORT records take one thread.
+constexpr int CCD_SORT = 4096, CCD_BLOCK = 256;
+struct CcdSort {
+    unsigned long long key[CCD_SORT];
+    int by_slot[CCD_SORT];     // record of each slot (body order)
+    int order[CCD_SORT];       // records in time-of-impact order
+    uint16_t place[CCD_SORT];  // slot -> place in that order
+    uint16_t hits[CCD_SORT];   // places of the records with a hit, in order
+    uint8_t moved[CCD_SORT];
+};
+__device__ void ccd_resolve_serial(DevWorld &w, int wd, int o0, int m) {
     CcdRec *rec = w.ccd;
-    for (int wd = blockIdx.x * blockDim.x + threadIdx.x; wd < w.num_worlds; wd += gridDim.x * blockDim.x) {
+    int *seg = w.ccd_seg + o0;
+    heap_sort(seg, m, [&](int x, int y) { return rec[x].body < rec[y].body; });
+    for (int k = 0; k < m; k++) rec[seg[k]].slot = k;
+    heap_sort(seg, m, [&](int x, int y) {
+        if (rec[x].fps != rec[y].fps) return rec[x].fps < rec[y].fps;
+        return rec[x].body < rec[y].body;
+    });
+    float2 lam = w.ccd_lambda[wd];
+    for (int k = 0; k < m; k++) {
+        CcdRec &c = rec[seg[k]];
+        if (c.hit >= 0) {
+            const int bi = w.ccd_index[c.hit];
+            ccd_hit(w, c, bi >= 0 ? &rec[seg[rec[bi].slot]] : nullptr, lam);
+        } else {
+            ccd_move(w, c, 1.f);
+        }
+    }
+    w.ccd_lambda[wd] = lam;
+}
+__global__ void __launch_bounds__(CCD_BLOCK) k_ccd_resolve(DevWorld w) {
+    if (w.ctr->num_ccd == 0) return;
+    extern __shared__ __align__(16) unsigned char ccd_smem[];
+    __shared__ int s_hits;
+    CcdSort &S = *reinterpret_cast<CcdSort *>(ccd_smem);
+    CcdRec *rec = w.ccd;
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int wd = blockIdx.x; wd < w.num_worlds; wd += gridDim.x) {
         const int o0 = w.ccd_world_off[wd], m = w.ccd_world_off[wd + 1] - o0;
         if (m <= 0) continue;
-        int *seg = w.ccd_seg + o0;
-        heap_sort(seg, m, [&](int x, int y) { return rec[x].body < rec[y].body; });
-        for (int k = 0; k < m; k++) rec[seg[k]].slot = k;
-        heap_sort(seg, m, [&](int x, int y) {
-            if (rec[x].fps != rec[y].fps) return rec[x].fps < rec[y].fps;
-            return rec[x].body < rec[y].body;
-        });
-        float2 lam = w.ccd_lambda[wd];
-        for (int k = 0; k < m; k++) {
-            CcdRec &c = rec[seg[k]];
-            const int a = c.body;
-            float move = 1.f;  // no hit: the whole displacement
-            if (c.hit >= 0) {
-                const int b = c.hit;
-                const int bi = w.ccd_index[b];
+        if (m > CCD_SORT) {
+            if (tid == 0) ccd_resolve_serial(w, wd, o0, m);
+            continue;
+        }
+        const int *seg = w.ccd_seg + o0;
+        int P = 2;
+        while (P < m) P <<= 1;
+        auto sort = [&]() {  // bitonic, the keys are distinct (the padding apart)
+            for (int kk = 2; kk <= P; kk <<= 1)
+                for (int j = kk >> 1; j > 0; j >>= 1) {
+                    for (int i = tid; i < P; i += CCD_BLOCK) {
+                        const int l = i ^ j;
+                        if (l > i && ((S.key[i] > S.key[l]) == ((i & kk) == 0))) {
+                            const unsigned long long t = S.key[i];
+                            S.key[i] = S.key[l];
+                            S.key[l] = t;
+                        }
+                    }
+                    __syncthreads();
+                }
+        };
+        for (int k = tid; k < P; k += CCD_BLOCK)
+            S.key[k] = k < m ? (unsigned long long)(unsigned)rec[seg[k]].body << 32 | (unsigned)seg[k] : ~0ull;
+        __syncthreads();
+        sort();
+        for (int k = tid; k < m; k += CCD_BLOCK) {
+            const int r = (int)(unsigned)S.key[k];
+            S.by_slot[k] = r;
+            rec[r].slot = k;
+            S.moved[k] = 0;
+            // (fps, body): the fraction's bits in the order of the floats, then the slot
+            const unsigned f = __float_as_uint(rec[r].fps + 0.f);
+            S.key[k] = (unsigned long long)(f & 0x80000000u ? ~f : f | 0x80000000u) << 32 | (unsigned)k;
+        }
+        __syncthreads();
+        sort();
+        for (int k = tid; k < m; k += CCD_BLOCK) {
+            const int slot = (int)(unsigned)S.key[k], r = S.by_slot[slot];
+            S.order[k] = r;
+            S.place[slot] = (uint16_t)k;
+            if (rec[r].hit >= 0) S.moved[k] = 2;  // a hit to resolve
+        }
+        __syncthreads();
+        if (tid < 32) {
+            int n = 0;
+            for (int k0 = 0; k0 < m; k0 += 32) {
+                const bool h = k0 + lane < m && S.moved[k0 + lane] == 2;
+                const unsigned b = __ballot_sync(0xffffffffu, h);
+                if (h) {
+                    S.hits[n + __popc(b & ((1u << lane) - 1u))] = (uint16_t)(k0 + lane);
+                    S.moved[k0 + lane] = 0;
+                }
+                n += __popc(b);
+            }
+            if (lane == 0) s_hits = n;
+        }
+        __syncthreads();
+        if (tid == 0 && s_hits > 0) {
+            float2 lam = w.ccd_lambda[wd];
+            for (int h = 0; h < s_hits; h++) {
+                const int k = S.hits[h];
+                CcdRec &c = rec[S.order[k]];
+                if (c.hit < 0) continue;  // a cascade took the hit: it moves on
+                const int bi = w.ccd_index[c.hit];
                 if (bi >= 0) {
-                    CcdRec &cb = rec[seg[rec[bi].slot]];
-                    if (cb.hit >= 0 && cb.point.w > c.point.w) {
-                        cb.hit = -1;
-                        cb.fps = c.point.w;
+                    const int kb = S.place[rec[bi].slot];
+                    if (kb < k && !S.moved[kb]) {  // its turn was before this one
+                        ccd_move(w, rec[bi], 1.f);
+                        S.moved[kb] = 1;
                     }
                 }
-                ccd_apply(w, c, a, b, lam);
-                move = c.fps;
-                if (sleeping_of(w.flags[b])) {
-                    w.flags[b] &= ~F_SLEEPING;
-                    reset_sleep(w, b);
-                }
+                ccd_hit(w, c, bi >= 0 ? &rec[S.order[rec[bi].slot]] : nullptr, lam);
+                S.moved[k] = 1;
             }
-            const uint32_t fa = w.flags[a];
-            const float3 p = xyz(w.pos[a]) + xyz(c.delta) * move;
-            const float3 cm = p + qrot(w.quat[a], shape_com(w, a, fa, w.shape[a]));
-            w.pos[a] = make_float4(p.x, p.y, p.z, 0.f);
-            w.com[a] = make_float4(cm.x, cm.y, cm.z, 0.f);
+            w.ccd_lambda[wd] = lam;
         }
-        w.ccd_lambda[wd] = lam;
+        __syncthreads();
+        for (int k = tid; k < m; k += CCD_BLOCK)
+            if (!S.moved[k]) ccd_move(w, rec[S.order[k]], 1.f);
+        __syncthreads();
     }
 }
 
@@ -2359,7 +2467,12 @@ void launch_ccd(DevWorld &w, float dt, cudaStream_t s) {
                        w.ccd_scan_tmp, s);
     cudaMemsetAsync(w.ccd_world_fill, 0, sizeof(int) * (size_t)w.num_worlds, s);
     k_ccd_scatter<<<grid_for(w.n, 256), 256, 0, s>>>(w);
-    k_ccd_resolve<<<grid_for(w.num_worlds, 64), 64, 0, s>>>(w);
+    static bool attr_set = false;  // set on the first (eager) step, before any graph capture
+    if (!attr_set) {
+        cudaFuncSetAttribute(k_ccd_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CcdSort));
+        attr_set = true;
+    }
+    k_ccd_resolve<<<std::min(w.num_worlds, 2 * device_sm_count()), CCD_BLOCK, sizeof(CcdSort), s>>>(w);
 }
 
 // blocks of the giant-island launch: one per SM, fewer if the kernel cannot be resident at that
