@@ -3429,6 +3429,20 @@ __device__ void ccd_cast_mesh(const DevWorld &w, uint32_t fa, float4 sa, float3 
         const float3 lo = f3(fminf(start.x, end.x) - r, fminf(start.y, end.y) - r, fminf(start.z, end.z) - r);
         const float3 hi = f3(fmaxf(start.x, end.x) + r, fmaxf(start.y, end.y) + r, fmaxf(start.z, end.z) + r);
         const float3 qc = (lo + hi) * 0.5f;
+        // The reference walks every node that meets the swept box (a 70 m diagonal sweep meets half
+        // a terrain).  A triangle can only be hit while the sphere's centre is within the radius of
+        // it, so nodes that the centre's path, grown by `reach`, misses or enters past the best
+        // hit hold no hit and are skipped; the rest are visited in the same order.  reach is the
+        // radius and the error of the tests below: their squared distances carry rounding errors of
+        // about 2^-24 of the squared lengths they subtract, bounded here with a factor of 64 to
+        // spare.  The mesh pass of 16,384 sweeps of 40-100 m over a 160 x 160-cell
+        // terrain: 20.5 -> 2.6 ms (a sphere's sweep had tested thousands of triangles).
+        const float len = sqrtf(lensq3(dInB));
+        const float3 rdir = len > 1e-10f ? dInB * (1.f / len) : f3(0.f, 0.f, 0.f);
+        const float far = len + sqrtf(lensq3(f3(fmaxf(fabsf(start.x), fabsf(end.x)), fmaxf(fabsf(start.y), fabsf(end.y)),
+                                                fmaxf(fabsf(start.z), fabsf(end.z)))));
+        const float reach = sqrtf(r * r + 1.6e-5f * (len + r) * (len + r)) + 4e-6f * far;
+        const float3 rv = f3(reach, reach, reach);
         // castSphereVsTriangleMeshAddHit :1781-1868: the penetration axis is the negated contact normal
         uint32_t tsub = 0xffffffffu;
         auto emit = [&](float fraction, float3 cp, float3 cn) {
@@ -3440,6 +3454,8 @@ __device__ void ccd_cast_mesh(const DevWorld &w, uint32_t fa, float4 sa, float3 
             const int node = stack[--sp];
             const float4 nlo = nodes[2 * node], nhi = nodes[2 * node + 1];
             if (!node_hits_box(nlo, nhi, lo, hi)) continue;
+            const float enter = ray_box_entry(start, rdir, len, xyz(nlo) - rv, xyz(nhi) + rv);
+            if (!(enter <= fmaf(fps, len, reach))) continue;
             const int aux = __float_as_int(nlo.w), tag = __float_as_int(nhi.w);
             if (tag >= 0) {
                 const int left = node + 1, right = aux;
@@ -4325,8 +4341,9 @@ void launch_collide_points(DevWorld &w, const float4 *pts, int np, const DevRayF
 // bodies from PASS 1's hits, as the ray queries do.  MODE picks the collector of
 // cast-shape-vs-shape.ts:165-226 as for the rays: the closest hit, the first hit found, or every
 // hit (one per convex body, one per mesh triangle) appended to hits[k * cap ...].
+constexpr int CAST_BLOCK = 32;  // one warp a block: a batch's few hundred warps spread over all SMs
 template <int PASS, int MODE>
-__global__ void __launch_bounds__(128, 4) k_cast_shapes(DevWorld w, const int2 *node_world, const DevShapeCast *qs,
+__global__ void __launch_bounds__(CAST_BLOCK, 16) k_cast_shapes(DevWorld w, const int2 *node_world, const DevShapeCast *qs,
                                                      int nq, DevRayFilter flt, DevShapeCastHit *hits, int cap,
                                                      int *counts) {
     const int n = w.n;
@@ -4934,10 +4951,10 @@ template <int MODE>
 static void cast_shapes_mode(DevWorld &w, const DevShapeCast *qs, int nq, const DevRayFilter &f, DevShapeCastHit *hits,
                              int cap, int *counts, cudaStream_t s) {
     if (w.num_mesh_bodies > 0) {
-        k_cast_shapes<1, MODE><<<grid_for(nq, 128, 16), 128, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
-        k_cast_shapes<2, MODE><<<grid_for(nq, 128, 16), 128, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
+        k_cast_shapes<1, MODE><<<grid_for(nq, CAST_BLOCK, 64), CAST_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
+        k_cast_shapes<2, MODE><<<grid_for(nq, CAST_BLOCK, 64), CAST_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
     } else {
-        k_cast_shapes<0, MODE><<<grid_for(nq, 128, 16), 128, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
+        k_cast_shapes<0, MODE><<<grid_for(nq, CAST_BLOCK, 64), CAST_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
     }
 }
 void launch_cast_shapes(DevWorld &w, const DevShapeCast *qs, int nq, const DevRayFilter &f, DevShapeCastHit *hits,
