@@ -13,6 +13,7 @@
 // body's AABB grown by the speculative contact distance, dbvt.ts:669 and
 // broadphase.ts:249) so the reported pair set equals the reference's.
 #include "cc_internal.cuh"
+#include "cc_sort_small.cuh"
 
 namespace cc {
 
@@ -92,34 +93,24 @@ __device__ void exact_aabb(float4 p4, float4 q4, const double lo[3], const doubl
     double m0 = ds(ds(1.0, yy), zz), m1 = da(yx, wz), m2 = ds(zx, wy);
     double m4 = ds(yx, wz), m5 = ds(ds(1.0, xx), zz), m6 = da(zy, wx);
     double m8 = da(zx, wy), m9 = ds(zy, wx), m10 = ds(ds(1.0, xx), yy);
-    double px = p4.x, py = p4.y, pz = p4.z;
-    double xs[2] = {lo[0], hi[0]}, ys[2] = {lo[1], hi[1]}, zs[2] = {lo[2], hi[2]};
-    double mnx = 0, mny = 0, mnz = 0, mxx = 0, mxy = 0, mxz = 0;
+    // The least and the greatest of the eight corners' sums ((m0 x + m4 y) + m8 z) + p, each
+    // operation rounded: rounding keeps the order, so the least sum is the sum of the least
+    // terms, and the term of an axis is least at the end that the sign of its factor picks.  18
+    // products and 18 sums in place of 60 sums and 42 FP64 comparisons: the kernel is bound by
+    // the FP64 pipe (511,195 bodies: 177 us with every corner, 86 us so).
+    const double m[3][3] = {{m0, m4, m8}, {m1, m5, m9}, {m2, m6, m10}}, p[3] = {p4.x, p4.y, p4.z};
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        double cx = xs[c & 1], cy = ys[(c >> 1) & 1], cz = zs[(c >> 2) & 1];
-        double wxv = da(da(da(dm(m0, cx), dm(m4, cy)), dm(m8, cz)), px);
-        double wyv = da(da(da(dm(m1, cx), dm(m5, cy)), dm(m9, cz)), py);
-        double wzv = da(da(da(dm(m2, cx), dm(m6, cy)), dm(m10, cz)), pz);
-        if (c == 0) {
-            mnx = mxx = wxv;
-            mny = mxy = wyv;
-            mnz = mxz = wzv;
-        } else {
-            mnx = fmin(mnx, wxv);
-            mny = fmin(mny, wyv);
-            mnz = fmin(mnz, wzv);
-            mxx = fmax(mxx, wxv);
-            mxy = fmax(mxy, wyv);
-            mxz = fmax(mxz, wzv);
+    for (int k = 0; k < 3; k++) {
+        double t_lo[3], t_hi[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const bool neg = __double2hiint(m[k][c]) < 0;
+            t_lo[c] = dm(m[k][c], neg ? hi[c] : lo[c]);
+            t_hi[c] = dm(m[k][c], neg ? lo[c] : hi[c]);
         }
+        out[k] = da(da(da(t_lo[0], t_lo[1]), t_lo[2]), p[k]);
+        out[3 + k] = da(da(da(t_hi[0], t_hi[1]), t_hi[2]), p[k]);
     }
-    out[0] = mnx;
-    out[1] = mny;
-    out[2] = mnz;
-    out[3] = mxx;
-    out[4] = mxy;
-    out[5] = mxz;
 }
 
 // local bounds of the shape in FP64 (box.ts:77-84, sphere.ts, capsule.ts:84-94)
@@ -239,20 +230,32 @@ __device__ __forceinline__ unsigned int expand_bits10(unsigned int v) {
     return v;
 }
 
-__global__ void k_morton(DevWorld w, const unsigned int *scene) {
-    float3 smin = f3(ord2f(scene[0]), ord2f(scene[1]), ord2f(scene[2]));
+// the scene bounds' origin and the scale to the Morton grid
+struct MortonGrid {
+    float3 smin, inv;
+};
+__device__ __forceinline__ MortonGrid morton_grid(const unsigned int *scene) {
+    MortonGrid g;
+    g.smin = f3(ord2f(scene[0]), ord2f(scene[1]), ord2f(scene[2]));
     float3 smax = f3(ord2f(scene[3]), ord2f(scene[4]), ord2f(scene[5]));
-    float3 ext = smax - smin;
-    float3 inv = f3(ext.x > 0.f ? 1023.f / ext.x : 0.f, ext.y > 0.f ? 1023.f / ext.y : 0.f,
-                    ext.z > 0.f ? 1023.f / ext.z : 0.f);
+    float3 ext = smax - g.smin;
+    g.inv = f3(ext.x > 0.f ? 1023.f / ext.x : 0.f, ext.y > 0.f ? 1023.f / ext.y : 0.f,
+               ext.z > 0.f ? 1023.f / ext.z : 0.f);
+    return g;
+}
+__device__ __forceinline__ unsigned long long morton_key(const DevWorld &w, const MortonGrid &g, int i) {
+    float3 c = (xyz(w.aabb_lo[i]) + xyz(w.aabb_hi[i])) * 0.5f;
+    float3 t = (c - g.smin);
+    unsigned int qx = (unsigned int)fminf(fmaxf(t.x * g.inv.x, 0.f), 1023.f);
+    unsigned int qy = (unsigned int)fminf(fmaxf(t.y * g.inv.y, 0.f), 1023.f);
+    unsigned int qz = (unsigned int)fminf(fmaxf(t.z * g.inv.z, 0.f), 1023.f);
+    unsigned int m = (expand_bits10(qx) << 2) | (expand_bits10(qy) << 1) | expand_bits10(qz);
+    return ((unsigned long long)(unsigned int)w.world[i] << 30) | m;
+}
+__global__ void k_morton(DevWorld w, const unsigned int *scene) {
+    const MortonGrid g = morton_grid(scene);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.n; i += gridDim.x * blockDim.x) {
-        float3 c = (xyz(w.aabb_lo[i]) + xyz(w.aabb_hi[i])) * 0.5f;
-        float3 t = (c - smin);
-        unsigned int qx = (unsigned int)fminf(fmaxf(t.x * inv.x, 0.f), 1023.f);
-        unsigned int qy = (unsigned int)fminf(fmaxf(t.y * inv.y, 0.f), 1023.f);
-        unsigned int qz = (unsigned int)fminf(fmaxf(t.z * inv.z, 0.f), 1023.f);
-        unsigned int m = (expand_bits10(qx) << 2) | (expand_bits10(qy) << 1) | expand_bits10(qz);
-        w.morton[i] = ((unsigned long long)(unsigned int)w.world[i] << 30) | m;
+        w.morton[i] = morton_key(w, g, i);
         w.order[i] = i;
     }
 }
@@ -267,29 +270,35 @@ __device__ __forceinline__ int lcp(const unsigned long long *k, int n, int i, in
     return __clzll(a ^ b);
 }
 
+// internal node i over the sorted keys: its children and the key range [first, last] it covers
+__device__ __forceinline__ void lbvh_node(const unsigned long long *k, int n, int i, int &left, int &right, int &first,
+                                          int &last) {
+    int d = (lcp(k, n, i, i + 1) - lcp(k, n, i, i - 1)) >= 0 ? 1 : -1;
+    int dmin = lcp(k, n, i, i - d);
+    int lmax = 2;
+    while (lcp(k, n, i, i + lmax * d) > dmin) lmax <<= 1;
+    int l = 0;
+    for (int t = lmax >> 1; t >= 1; t >>= 1)
+        if (lcp(k, n, i, i + (l + t) * d) > dmin) l += t;
+    int j = i + l * d;
+    int dnode = lcp(k, n, i, j);
+    int s = 0;
+    int div = 2;
+    for (int t = (l + div - 1) / div; t >= 1; div <<= 1, t = (l + div - 1) / div) {
+        if (lcp(k, n, i, i + (s + t) * d) > dnode) s += t;
+        if (t == 1) break;
+    }
+    int gamma = i + s * d + min(d, 0);
+    first = min(i, j), last = max(i, j);
+    left = (first == gamma) ? (n - 1 + gamma) : gamma;
+    right = (last == gamma + 1) ? (n - 1 + gamma + 1) : gamma + 1;
+}
 __global__ void k_lbvh_build(DevWorld w, int2 *node_world) {
     int n = w.n;
     const unsigned long long *k = w.morton;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
-        int d = (lcp(k, n, i, i + 1) - lcp(k, n, i, i - 1)) >= 0 ? 1 : -1;
-        int dmin = lcp(k, n, i, i - d);
-        int lmax = 2;
-        while (lcp(k, n, i, i + lmax * d) > dmin) lmax <<= 1;
-        int l = 0;
-        for (int t = lmax >> 1; t >= 1; t >>= 1)
-            if (lcp(k, n, i, i + (l + t) * d) > dmin) l += t;
-        int j = i + l * d;
-        int dnode = lcp(k, n, i, j);
-        int s = 0;
-        int div = 2;
-        for (int t = (l + div - 1) / div; t >= 1; div <<= 1, t = (l + div - 1) / div) {
-            if (lcp(k, n, i, i + (s + t) * d) > dnode) s += t;
-            if (t == 1) break;
-        }
-        int gamma = i + s * d + min(d, 0);
-        int first = min(i, j), last = max(i, j);
-        int left = (first == gamma) ? (n - 1 + gamma) : gamma;
-        int right = (last == gamma + 1) ? (n - 1 + gamma + 1) : gamma + 1;
+        int left, right, first, last;
+        lbvh_node(k, n, i, left, right, first, last);
         w.node_child[i] = make_int2(left, right);
         w.node_parent[left] = i;
         w.node_parent[right] = i;
@@ -297,6 +306,72 @@ __global__ void k_lbvh_build(DevWorld w, int2 *node_world) {
         node_world[i] = make_int2((int)(k[first] >> 30), (int)(k[last] >> 30));
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) w.node_parent[n == 1 ? 0 : 0] = -1;
+}
+
+// Few bodies: Morton keys, sort, tree and bounds in one block.  The keys, the links and the arrival
+// flags stay in shared memory; a climbing thread keeps its node's bounds in registers and reads the
+// sibling's.  One launch in place of 23 to 33 (a 32-body world: 105 -> 17 us, measured one by one),
+// up to a body per thread: at 7,518 bodies it takes 168 us, the tree's own kernels after a sort in
+// one block 90 us.
+constexpr int TREE_SMALL = SORT_BLOCK;
+__global__ void __launch_bounds__(SORT_BLOCK) k_tree_small(DevWorld w, const unsigned int *scene, int2 *node_world,
+                                                           int bits) {
+    extern __shared__ __align__(16) unsigned char tree_smem[];
+    const int n = w.n, tid = threadIdx.x;
+    SmallSort S(tree_smem, n);
+    const MortonGrid g = morton_grid(scene);
+    for (int i = tid; i < n; i += SORT_BLOCK) {
+        S.key[0][i] = morton_key(w, g, i);
+        S.val[0][i] = (uint16_t)i;
+    }
+    const int b = S.sort(n, bits);
+    const unsigned long long *key = S.key[b];
+    const uint16_t *order = S.val[b];
+    constexpr unsigned NONE = 0xffffu;
+    uint16_t *parent = (uint16_t *)S.key[b ^ 1], *child = parent + 2 * n;  // 2n - 1 nodes; 2 per internal node
+    unsigned *arrived = (unsigned *)S.count;                               // a bit per internal node
+    for (int k = tid; k < (n + 31) / 32; k += SORT_BLOCK) arrived[k] = 0;
+    for (int j = tid; j < n; j += SORT_BLOCK) {
+        w.morton[j] = key[j];
+        w.order[j] = order[j];
+    }
+    for (int i = tid; i < n - 1; i += SORT_BLOCK) {
+        int left, right, first, last;
+        lbvh_node(key, n, i, left, right, first, last);
+        w.node_child[i] = make_int2(left, right);
+        w.node_parent[left] = i;
+        w.node_parent[right] = i;
+        child[2 * i] = (uint16_t)left;
+        child[2 * i + 1] = (uint16_t)right;
+        parent[left] = parent[right] = (uint16_t)i;
+        node_world[i] = make_int2((int)(key[first] >> 30), (int)(key[last] >> 30));
+    }
+    if (tid == 0) {
+        w.node_parent[0] = -1;
+        parent[0] = (uint16_t)NONE;  // the root (or the only leaf)
+    }
+    __syncthreads();
+    for (int j = tid; j < n; j += SORT_BLOCK) {
+        const int body = order[j];
+        int node = n - 1 + j;
+        float4 lo = w.aabb_lo[body], hi = w.aabb_hi[body];
+        w.node_lo[node] = lo;
+        w.node_hi[node] = hi;
+        const int wd = w.world[body];
+        node_world[node] = make_int2(wd, wd);
+        for (unsigned p = parent[node]; p != NONE; p = parent[p]) {
+            __threadfence_block();
+            if (!(atomicOr(&arrived[p >> 5], 1u << (p & 31)) >> (p & 31) & 1u)) break;  // first child to arrive stops
+            __threadfence_block();
+            const int cx = child[2 * p], sib = cx == node ? child[2 * p + 1] : cx;
+            const float4 sl = w.node_lo[sib], sh = w.node_hi[sib];
+            lo = make_float4(fminf(lo.x, sl.x), fminf(lo.y, sl.y), fminf(lo.z, sl.z), 0.f);
+            hi = make_float4(fmaxf(hi.x, sh.x), fmaxf(hi.y, sh.y), fmaxf(hi.z, sh.z), 0.f);
+            node = (int)p;
+            w.node_lo[node] = lo;
+            w.node_hi[node] = hi;
+        }
+    }
 }
 
 __global__ void k_lbvh_refit(DevWorld w, int2 *node_world, const int *gate) {
@@ -512,16 +587,32 @@ void launch_ccd_bounds(DevWorld &w, float dt, cudaStream_t s) {
     k_lbvh_refit<<<grid_for(n, 256), 256, 0, s>>>(w, w.node_world, &w.ctr->num_ccd);
 }
 
-void launch_broadphase(DevWorld &w, cudaStream_t s) {
-    int n = w.n;
+// the bodies' boxes and the tree over them
+static void launch_tree(DevWorld &w, cudaStream_t s) {
+    const int n = w.n;
     k_reset_scene<<<1, 32, 0, s>>>(w.scene);
-    k_update_bounds<<<grid_for(n, 256), 256, 0, s>>>(w, w.scene);
-    k_morton<<<grid_for(n, 256), 256, 0, s>>>(w, w.scene);
+    k_update_bounds<<<grid_for(n, 64), 64, 0, s>>>(w, w.scene);
     int wbits = 0;
     while ((1 << wbits) < w.num_worlds) wbits++;
+    if (n <= TREE_SMALL) {
+        static bool attr_set = false;  // set on the first (eager) step, before any graph capture
+        if (!attr_set) {
+            cudaFuncSetAttribute(k_tree_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SmallSort::bytes(TREE_SMALL));
+            attr_set = true;
+        }
+        k_tree_small<<<1, SORT_BLOCK, SmallSort::bytes(n), s>>>(w, w.scene, w.node_world, 30 + wbits);
+        return;
+    }
+    k_morton<<<grid_for(n, 256), 256, 0, s>>>(w, w.scene);
     radix_sort_pairs_u64(w.morton, w.morton_alt, w.order, w.order_alt, n, 30 + wbits, w.scan_tmp, s);
-    if (n > 1) k_lbvh_build<<<grid_for(n - 1, 256), 256, 0, s>>>(w, w.node_world);
+    k_lbvh_build<<<grid_for(n - 1, 256), 256, 0, s>>>(w, w.node_world);
     k_lbvh_refit<<<grid_for(n, 256), 256, 0, s>>>(w, w.node_world, nullptr);
+}
+
+void launch_broadphase(DevWorld &w, cudaStream_t s) {
+    int n = w.n;
+    launch_tree(w, s);
     k_find_pairs<<<grid_for(n, 128, 16), 128, 0, s>>>(w, w.node_world);
 }
 
@@ -556,16 +647,7 @@ void launch_ray_order(DevWorld &w, const DevRay *rays, int nr, unsigned long lon
 
 // the broadphase without its pair search: current boxes, Morton order and tree
 void launch_query_tree(DevWorld &w, cudaStream_t s) {
-    int n = w.n;
-    if (n == 0) return;
-    k_reset_scene<<<1, 32, 0, s>>>(w.scene);
-    k_update_bounds<<<grid_for(n, 256), 256, 0, s>>>(w, w.scene);
-    k_morton<<<grid_for(n, 256), 256, 0, s>>>(w, w.scene);
-    int wbits = 0;
-    while ((1 << wbits) < w.num_worlds) wbits++;
-    radix_sort_pairs_u64(w.morton, w.morton_alt, w.order, w.order_alt, n, 30 + wbits, w.scan_tmp, s);
-    if (n > 1) k_lbvh_build<<<grid_for(n - 1, 256), 256, 0, s>>>(w, w.node_world);
-    k_lbvh_refit<<<grid_for(n, 256), 256, 0, s>>>(w, w.node_world, nullptr);
+    if (w.n > 0) launch_tree(w, s);
 }
 
 }  // namespace cc

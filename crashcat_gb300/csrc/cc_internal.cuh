@@ -511,6 +511,7 @@ struct DevWorld {
     cudaStream_t aux3_stream;  // fourth stream: the per-warp solve of the islands past 32 contacts
     cudaStream_t aux4_stream;  // fifth stream: the larger instance of the per-CTA solve
     cudaEvent_t ev_fork, ev_join, ev_join2, ev_join3, ev_join4;
+    int small_island_max;    // DevSettings::small_island_max_cons, for the choice of launches
     int warp_blocks_per_sm;  // launch shape of the per-warp island solve
     int warp_carveout;       // shared-memory carveout (percent) of the per-warp island solve
     // persistent contact cache (double buffered by parity)
@@ -929,6 +930,8 @@ constexpr int GIANT_COLOURS = 1024;    // colours of the giant-island solve; the
 
 // scan / sort utilities (cc_scan.cu)
 void exclusive_scan_int(const int *in, int *out, int n, int *total, int *tmp, cudaStream_t s);
+void exclusive_scan_multi(const int *in0, int *out0, const int *in1, int *out1, const int *in2, int *out2, int n,
+                          int *tmp, cudaStream_t s);
 void radix_sort_pairs_u64(unsigned long long *keys, unsigned long long *keys_alt, int *vals, int *vals_alt, int n,
                           int bits, int *tmp, cudaStream_t s, const int *n_dev = nullptr);
 size_t scan_tmp_ints(int n);

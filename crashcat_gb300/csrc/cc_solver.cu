@@ -2069,9 +2069,8 @@ void launch_contacts_and_islands(DevWorld &w, float dt, float, cudaStream_t s) {
     k_uf_roots<<<grid_for(w.n, 256), 256, 0, s>>>(w, w.root_flag);
     exclusive_scan_int(w.root_flag, w.island_id_of_root, w.n, &w.ctr->num_islands, w.scan_tmp, s);
     k_island_count<<<grid_for(nmax, 256), 256, 0, s>>>(w, w.island_id_of_root);
-    exclusive_scan_int(w.island_body_count, w.island_body_off, w.n, nullptr, w.scan_tmp, s);
-    exclusive_scan_int(w.island_cons_count, w.island_cons_off, w.n, nullptr, w.scan_tmp, s);
-    if (nj > 0) exclusive_scan_int(w.island_joint_count, w.island_joint_off, w.n, nullptr, w.scan_tmp, s);
+    exclusive_scan_multi(w.island_body_count, w.island_body_off, w.island_cons_count, w.island_cons_off,
+                         nj > 0 ? w.island_joint_count : nullptr, w.island_joint_off, w.n, w.scan_tmp, s);
     k_island_scatter<<<grid_for(nmax, 256), 256, 0, s>>>(w);
     k_island_classify<<<grid_for(w.n, 256), 256, 0, s>>>(w, w.small_list, w.large_list);
     if (nj > 0 && dt > 0.f) k_joint_setup<<<grid_for(nj, 128), 128, 0, s>>>(w, dt);
