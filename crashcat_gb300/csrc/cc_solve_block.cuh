@@ -569,26 +569,13 @@ __global__ void __launch_bounds__(T::THREADS, 1)
                 const float4 id = rows[ROW_ID * stride + tasks[first + (on ? lane : 0)]];
                 const float4 *c4 = (const float4 *)&w.cons[__float_as_int(id.y)];
                 const int4 hd = *(const int4 *)c4;
-                const float4 n4 = c4[1], m1 = c4[2], m2 = c4[3];
-                const int bits = __float_as_int(id.z), n = bits & 15;
-                float3 la3[4], lb3[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    la3[k] = lb3[k] = f3(0.f, 0.f, 0.f);
-                    if (k < n) {
-                        const float4 a = c4[6 + 5 * k], b = c4[7 + 5 * k];
-                        la3[k] = f3(a.z, a.w, b.x);
-                        lb3[k] = f3(b.y, b.z, b.w);
-                    }
-                }
+                const uint32_t fa = w.flags[hd.x], fb = w.flags[hd.y];
                 const unsigned la = __float_as_uint(id.x) & 0xffffu, lb = __float_as_uint(id.x) >> 16;
-                PoseSide SA{(bits >> 4) & 3, (bits >> 8) & 63, w.inertia_rot[hd.x], xyz(w.inv_inertia[hd.x]), m1.w};
-                PoseSide SB{(bits >> 6) & 3, (bits >> 16) & 63, w.inertia_rot[hd.y], xyz(w.inv_inertia[hd.y]), m2.w};
                 PoseRef PA, PB;
                 if (la == BLOCK_NONE) PA = PoseRef{xyz(w.com[hd.x]), w.quat[hd.x]};
                 if (lb == BLOCK_NONE) PB = PoseRef{xyz(w.com[hd.y]), w.quat[hd.y]};
                 if (!turn(dep)) break;
-                if (on && (SA.motion == DYNAMIC || SB.motion == DYNAMIC)) {
+                if (on) {
                     if (la != BLOCK_NONE) {
                         const float *s = state + 7 * la;
                         PA = PoseRef{f3(s[0], s[1], s[2]), make_float4(s[3], s[4], s[5], s[6])};
@@ -597,18 +584,9 @@ __global__ void __launch_bounds__(T::THREADS, 1)
                         const float *s = state + 7 * lb;
                         PB = PoseRef{f3(s[0], s[1], s[2]), make_float4(s[3], s[4], s[5], s[6])};
                     }
-                    const Mat3 RA = quat_to_mat(PA.q), RB = quat_to_mat(PB.q);
-                    Sym3 IA{0, 0, 0, 0, 0, 0}, IB{0, 0, 0, 0, 0, 0};
-                    if (SA.motion == DYNAMIC) IA = world_inv_inertia(PA.q, SA.inertia_rot, SA.inv_inertia, SA.dof);
-                    if (SB.motion == DYNAMIC) IB = world_inv_inertia(PB.q, SB.inertia_rot, SB.inv_inertia, SB.dof);
-                    bool applied = false;
-                    for (int k = 0; k < n; k++) {
-                        const float3 pa = k == 0 ? la3[0] : (k == 1 ? la3[1] : (k == 2 ? la3[2] : la3[3]));
-                        const float3 pb = k == 0 ? lb3[0] : (k == 1 ? lb3[1] : (k == 2 ? lb3[2] : lb3[3]));
-                        applied = position_point(pa, pb, xyz(n4), PA, PB, RA, RB, IA, IB, SA, SB) || applied;
-                    }
-                    if (applied) {
-                        if (la != BLOCK_NONE && SA.motion == DYNAMIC) {
+                    const ContactConstraint &con = w.cons[__float_as_int(id.y)];
+                    if (solve_position_con(w, con, PA, PB, motion_of(fa), motion_of(fb), fa, fb)) {
+                        if (la != BLOCK_NONE && motion_of(fa) == DYNAMIC) {
                             float *s = state + 7 * la;
                             s[0] = PA.com.x;
                             s[1] = PA.com.y;
@@ -618,7 +596,7 @@ __global__ void __launch_bounds__(T::THREADS, 1)
                             s[5] = PA.q.z;
                             s[6] = PA.q.w;
                         }
-                        if (lb != BLOCK_NONE && SB.motion == DYNAMIC) {
+                        if (lb != BLOCK_NONE && motion_of(fb) == DYNAMIC) {
                             float *s = state + 7 * lb;
                             s[0] = PB.com.x;
                             s[1] = PB.com.y;

@@ -20,6 +20,8 @@
 // into the last solver pass.
 #include <math_constants.h>
 
+#include <algorithm>
+
 #include "cc_internal.cuh"
 #include "cc_swing.cuh"
 
@@ -768,46 +770,7 @@ struct PoseRef {
     float4 q;
 };
 
-// one side of a contact in the position solve: the body's motion, degrees of freedom and local inertia
-struct PoseSide {
-    int motion, dof;
-    float4 inertia_rot;
-    float3 inv_inertia;
-    float im;
-};
-// position solve of one contact point (contact-constraints.ts:1098-1216) with the contact's
-// rotations and inverse inertias; returns true if an impulse was applied
-__device__ __forceinline__ bool position_point(float3 localA, float3 localB, float3 normal, PoseRef &PA, PoseRef &PB,
-                                               const Mat3 &RA, const Mat3 &RB, const Sym3 &IA, const Sym3 &IB,
-                                               const PoseSide &SA, const PoseSide &SB) {
-    float3 pa = PA.com + mmul(RA, localA);
-    float3 pb = PB.com + mmul(RB, localB);
-    float sep = dot3(pb - pa, normal) + c_settings.slop;
-    sep = fmaxf(sep, -c_settings.max_pen);
-    if (sep >= 0.f) return false;
-    float3 mid = (pa + pb) * 0.5f;
-    float3 rA = mid - PA.com, rB = mid - PB.com;
-    float iem = inv_eff_mass(SA.motion == DYNAMIC, SB.motion == DYNAMIC, SA.im, SB.im, IA, IB, rA, rB, normal);
-    if (iem == 0.f) return false;
-    float eff = 1.f / iem;
-    float lambda = -eff * c_settings.baumgarte * sep;
-    if (SA.motion == DYNAMIC) {
-        PA.com = PA.com - normal * (lambda * SA.im);
-        if (!(SA.dof & 1)) PA.com.x = 0.f;
-        if (!(SA.dof & 2)) PA.com.y = 0.f;
-        if (!(SA.dof & 4)) PA.com.z = 0.f;
-        PA.q = rotation_step(PA.q, -(symmul(IA, cross3(rA, normal)) * lambda));
-    }
-    if (SB.motion == DYNAMIC) {
-        PB.com = PB.com + normal * (lambda * SB.im);
-        if (!(SB.dof & 1)) PB.com.x = 0.f;
-        if (!(SB.dof & 2)) PB.com.y = 0.f;
-        if (!(SB.dof & 4)) PB.com.z = 0.f;
-        PB.q = rotation_step(PB.q, symmul(IB, cross3(rB, normal)) * lambda);
-    }
-    return true;
-}
-// position solve of one contact; returns true if an impulse was applied
+// position solve of one contact (contact-constraints.ts:1098-1216); returns true if an impulse was applied
 __device__ bool solve_position_con(DevWorld &w, const ContactConstraint &c, PoseRef &PA, PoseRef &PB, int ma, int mb,
                                    uint32_t fa, uint32_t fb) {
     if (ma != DYNAMIC && mb != DYNAMIC) return false;
@@ -815,11 +778,39 @@ __device__ bool solve_position_con(DevWorld &w, const ContactConstraint &c, Pose
     // rotations and inverse inertias are taken once per contact, as the reference does
     const Mat3 RA = quat_to_mat(PA.q), RB = quat_to_mat(PB.q);
     Sym3 IA{0, 0, 0, 0, 0, 0}, IB{0, 0, 0, 0, 0, 0};
-    PoseSide SA{ma, dof_of(fa), {}, {}, c.invMassA}, SB{mb, dof_of(fb), {}, {}, c.invMassB};
-    if (ma == DYNAMIC) IA = world_inv_inertia(PA.q, w.inertia_rot[c.a], xyz(w.inv_inertia[c.a]), SA.dof);
-    if (mb == DYNAMIC) IB = world_inv_inertia(PB.q, w.inertia_rot[c.b], xyz(w.inv_inertia[c.b]), SB.dof);
-    for (int k = 0; k < c.n; k++)
-        any = position_point(c.p[k].localA, c.p[k].localB, c.normal, PA, PB, RA, RB, IA, IB, SA, SB) || any;
+    if (ma == DYNAMIC) IA = world_inv_inertia(PA.q, w.inertia_rot[c.a], xyz(w.inv_inertia[c.a]), dof_of(fa));
+    if (mb == DYNAMIC) IB = world_inv_inertia(PB.q, w.inertia_rot[c.b], xyz(w.inv_inertia[c.b]), dof_of(fb));
+    for (int k = 0; k < c.n; k++) {
+        const ContactPoint &p = c.p[k];
+        float3 pa = PA.com + mmul(RA, p.localA);
+        float3 pb = PB.com + mmul(RB, p.localB);
+        float sep = dot3(pb - pa, c.normal) + c_settings.slop;
+        sep = fmaxf(sep, -c_settings.max_pen);
+        if (sep >= 0.f) continue;
+        float3 mid = (pa + pb) * 0.5f;
+        float3 rA = mid - PA.com, rB = mid - PB.com;
+        float iem = inv_eff_mass(ma == DYNAMIC, mb == DYNAMIC, c.invMassA, c.invMassB, IA, IB, rA, rB, c.normal);
+        if (iem == 0.f) continue;
+        float eff = 1.f / iem;
+        float lambda = -eff * c_settings.baumgarte * sep;
+        if (ma == DYNAMIC) {
+            PA.com = PA.com - c.normal * (lambda * c.invMassA);
+            int d = dof_of(fa);
+            if (!(d & 1)) PA.com.x = 0.f;
+            if (!(d & 2)) PA.com.y = 0.f;
+            if (!(d & 4)) PA.com.z = 0.f;
+            PA.q = rotation_step(PA.q, -(symmul(IA, cross3(rA, c.normal)) * lambda));
+        }
+        if (mb == DYNAMIC) {
+            PB.com = PB.com + c.normal * (lambda * c.invMassB);
+            int d = dof_of(fb);
+            if (!(d & 1)) PB.com.x = 0.f;
+            if (!(d & 2)) PB.com.y = 0.f;
+            if (!(d & 4)) PB.com.z = 0.f;
+            PB.q = rotation_step(PB.q, symmul(IB, cross3(rB, c.normal)) * lambda);
+        }
+        any = true;
+    }
     return any;
 }
 
@@ -964,11 +955,13 @@ __global__ void k_joint_setup(DevWorld w, float dt) {
 // ---------------------------------------------------------------------------
 // small islands: one thread runs the island in the reference's exact order
 // ---------------------------------------------------------------------------
-// JOINTS: the islands with joints (their own list); the contact-only instance carries no joint code
+__device__ __forceinline__ bool lanes_take(const DevWorld &w);
+// JOINTS: the islands with joints (their own list); the contact-only instance carries no joint code,
+// and leaves the islands to k_solve_lanes when they are few
 template <bool JOINTS>
 __global__ void __launch_bounds__(128) k_solve_small(DevWorld w, CacheTables ct, const int *small_list, float dt,
                                                       float ratio, int phase) {
-    if (islands_failed(w)) return;
+    if (islands_failed(w) || (!JOINTS && lanes_take(w))) return;
     int ns = JOINTS ? w.ctr->num_small_joint_islands : w.ctr->num_small_islands;
     CacheRecord *crecs = ct.recs[*ct.parity];
     // Islands without joints come by size, most contacts first, in chunks of 32: a warp's lanes
@@ -1092,6 +1085,7 @@ __global__ void __launch_bounds__(128) k_solve_small(DevWorld w, CacheTables ct,
 }
 
 #include "cc_solve_block.cuh"
+#include "cc_solve_lanes.cuh"
 
 // ---------------------------------------------------------------------------
 // large islands with joints: one CTA per island, contacts sorted by the reference key,
@@ -1456,7 +1450,7 @@ __device__ __forceinline__ void warp_store(WI &s, int local, const BodyRef &b) {
 template <class WI>
 __global__ void __launch_bounds__(WARP_BLOCK) k_solve_warp(DevWorld w, CacheTables ct, float dt, float ratio,
                                                             int phase, int b0, int b1, int *cursor) {
-    if (islands_failed(w)) return;
+    if (islands_failed(w) || (b0 == 0 && lanes_take(w))) return;
     extern __shared__ __align__(16) unsigned char warp_smem_raw[];  // WARPS_PER_BLOCK islands
     const int lane = threadIdx.x & 31;
     WI &S = reinterpret_cast<WI *>(warp_smem_raw)[threadIdx.x >> 5];
@@ -2094,7 +2088,13 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
         cudaStreamWaitEvent(w.aux2_stream, w.ev_fork, 0);
         s_small = w.aux2_stream;
     }
-    k_solve_small<false><<<grid_for(w.n, 128, 16), 128, 0, s_small>>>(w, ct, w.small_list, dt, ratio, phase);
+    // a world of few bodies has few islands: k_solve_lanes alone; else the step's count decides
+    const bool lanes = w.small_island_max < SMALL_BUCKETS, lanes_only = lanes && w.n <= LANE_ISLANDS;
+    if (!lanes_only)
+        k_solve_small<false><<<grid_for(w.n, 128, 16), 128, 0, s_small>>>(w, ct, w.small_list, dt, ratio, phase);
+    if (lanes)
+        k_solve_lanes<<<grid_for(std::min(w.n, LANE_ISLANDS), LANE_BLOCK / 32, 8), LANE_BLOCK, 0,
+                        s_small>>>(w, ct, w.small_list, dt, ratio, phase);
     if (joints)
         k_solve_small<true><<<grid_for(w.n, 128, 16), 128, 0, s_small>>>(w, ct, w.small_joint_list, dt, ratio,
                                                                         phase);
@@ -2162,7 +2162,8 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
     k_solve_warp<WarpIsland><<<device_sm_count() * w.warp_blocks_per_sm, WARP_BLOCK, warp_smem, w.aux3_stream>>>(
         w, ct, dt, ratio, phase, 2, MID_BUCKETS, &w.ctr->mid_cursor);
     cudaEventRecord(w.ev_join3, w.aux3_stream);
-    k_solve_warp<WarpIslandS><<<device_sm_count() * warp_s_blocks_per_sm, WARP_BLOCK, warp_s_smem, s>>>(
+    if (!lanes_only)
+        k_solve_warp<WarpIslandS><<<device_sm_count() * warp_s_blocks_per_sm, WARP_BLOCK, warp_s_smem, s>>>(
         w, ct, dt, ratio, phase, 0, 2, &w.ctr->mid_cursor_s);
     cudaStreamWaitEvent(s, w.ev_join, 0);
     cudaStreamWaitEvent(s, w.ev_join3, 0);

@@ -468,6 +468,7 @@ int cc_world_create(const cc_world_settings *s, cc_world **out) {
             int v = atoi(e);
             if (v >= 4 && v <= 32) w.epa_packed_points = v;
         }
+        w.small_island_max = d.small_island_max_cons;
         w.warp_blocks_per_sm = 4;
         w.warp_carveout = 50;
         if (const char *e = getenv("CRASHCAT_WARP_BLOCKS_PER_SM")) {
@@ -2039,7 +2040,7 @@ static int tune_apply(cc_world *W, const TuneShape &t) {
     w.epa_threads = blocks * 64;
     w.epa_fetch_warp = t.epa_lockstep;
     w.warp_blocks_per_sm = t.warp_blocks_per_sm;
-    W->dev_settings.small_island_max_cons = t.small_max;
+    W->dev_settings.small_island_max_cons = w.small_island_max = t.small_max;
     set_giant_min(w, t.giant_min);
     drop_graph(W);
     return CC_OK;
