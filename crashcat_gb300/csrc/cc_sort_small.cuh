@@ -4,7 +4,7 @@
 
 namespace cc {
 
-constexpr int SORT_BLOCK = 1024, SORT_WARPS = SORT_BLOCK / 32, SORT_SMALL = 8192;
+constexpr int SORT_BLOCK = 1024, SORT_WARPS = SORT_BLOCK / 32, SORT_SMALL = 9216;
 
 struct SmallSort {
     static constexpr int ITEMS = SORT_SMALL / SORT_BLOCK;  // keys per lane at most
