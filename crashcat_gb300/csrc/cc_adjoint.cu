@@ -501,7 +501,8 @@ __global__ void k_adj_islands(DevWorld w, TapeStep t, AdjBuffers a, float ratio,
     const int iters = c_settings.vel_iters;
     const size_t stride_it = (size_t)t.counts[0] * ROWS_PER_CON;
     const bool warm = c_settings.warm_starting != 0;
-    for (int isl = blockIdx.x * blockDim.x + threadIdx.x; isl < ni; isl += gridDim.x * blockDim.x) {
+    const Spread sp = spread_items(ni);
+    for (int isl = sp.first; isl < ni; isl += sp.step) {
         int off = t.isl_off[isl], nc = t.isl_cnt[isl];
         if (nc == 0) continue;
         int *ord = t.isl_cons + off;
@@ -699,7 +700,7 @@ void launch_adjoint_step(DevWorld &w, TapeStep &t, AdjBuffers &a, float dt, floa
     k_adj_begin<<<grid_for(w.n, 256), 256, 0, s>>>(w, t, a, dt);
     cudaMemsetAsync(out.keys, 0xff, sizeof(unsigned long long) * (size_t)w.cache_cap, s);
     cudaMemsetAsync(out.vals, 0, sizeof(float) * ROWS_PER_CON * (size_t)w.cache_cap, s);
-    k_adj_islands<<<grid_for(w.n, 64), 64, 0, s>>>(w, t, a, ratio, in, out);
+    k_adj_islands<<<spread_grid(w.n), SPREAD_BLOCK, 0, s>>>(w, t, a, ratio, in, out);
     k_adj_mu<<<grid_for(w.max_manifolds, 256), 256, 0, s>>>(w, t, a);
     k_adj_force<<<grid_for(w.n, 256), 256, 0, s>>>(w, t, a);
 }

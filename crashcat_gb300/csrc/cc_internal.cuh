@@ -807,6 +807,28 @@ inline int grid_for(int n, int block, int max_blocks_per_sm = 8) {
     return g;
 }
 
+// Items over the grid's warps for kernels whose items run on long, divergent paths.  Fewer items
+// than lanes: a warp takes a run of items on its first lanes, so that all SMs take part and the
+// lanes of a warp wait for few others' branches; consecutive runs go to different blocks.  At least
+// as many items as lanes: 32 a warp, neighbours in one block.  `share`: one warp in so many is
+// enough to fill the SMs.  for (i = sp.first; i < total; i += sp.step)
+struct Spread {
+    int first, step;
+};
+__device__ __forceinline__ Spread spread_items(int total, int share = 1) {
+    const int wpb = blockDim.x >> 5, warps = gridDim.x * wpb, lane = threadIdx.x & 31;
+    const int per = max(1, (int)(((long long)total * share + warps - 1) / warps));
+    if (per >= 32) return Spread{(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x)};
+    const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    return Spread{lane < per ? warp * per + lane : total, warps * per};
+}
+// blocks of one warp for `items` items at most: up to 16 warps per SM
+constexpr int SPREAD_BLOCK = 32;
+inline int spread_grid(int items) {
+    const int cap = device_sm_count() * 16;
+    return items < 1 ? 1 : (items < cap ? items : cap);
+}
+
 // host launchers implemented in the .cu files
 void launch_integrate_forces(DevWorld &w, float dt, cudaStream_t s);
 void launch_broadphase(DevWorld &w, cudaStream_t s);

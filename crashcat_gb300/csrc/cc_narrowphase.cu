@@ -1146,7 +1146,8 @@ __global__ void k_pair_order(DevWorld w) {
 template <bool HULLS>
 __global__ void __launch_bounds__(128) k_narrowphase(DevWorld w, EpaItem *epa_items) {
     int np = min(w.ctr->num_pairs, w.max_pairs);
-    for (int pk = blockIdx.x * blockDim.x + threadIdx.x; pk < np; pk += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(np, 4);
+    for (int pk = spread.first; pk < np; pk += spread.step) {
         const int pi = w.pair_order[pk];  // grouped by collide class
         int2 pr = w.pairs[pi];
         int a = pr.x, b = pr.y;
@@ -2428,7 +2429,8 @@ __global__ void __launch_bounds__(EPA_BIG_BLOCK) k_epa_big(DevWorld w, EpaItem *
 template <bool HULLS>
 __global__ void __launch_bounds__(128) k_epa_emit(DevWorld w, const EpaItem *items) {
     int ne = min(w.ctr->num_epa, w.max_epa);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(ne, 4);
+    for (int i = spread.first; i < ne; i += spread.step) {
         const EpaItem &it = items[i];
         if (it.size != 1 || it.tri >= 0) continue;
         bool hull = shape_of(w.flags[it.a]) == SHAPE_HULL || shape_of(w.flags[it.b]) == SHAPE_HULL;
@@ -2991,7 +2993,8 @@ __device__ void mesh_pair(DevWorld &w, EpaItem *epa_items, int k, MeshReduceT<M>
 template <int PASS>
 __global__ void __launch_bounds__(64) k_mesh_narrowphase(DevWorld w, EpaItem *epa_items) {
     const int npairs = min(w.ctr->num_mesh_pairs, w.max_pairs);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < npairs; k += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(npairs);
+    for (int k = spread.first; k < npairs; k += spread.step) {
         MeshReduce red;
         mesh_pair<PASS, MESH_MAXM>(w, epa_items, k, red);
     }
@@ -3176,9 +3179,9 @@ __global__ void __launch_bounds__(64) k_compound_pairs(DevWorld w) {
 void launch_mesh_narrowphase(DevWorld &w, int pass, cudaStream_t s) {
     EpaItem *items = (EpaItem *)w.epa_items;
     if (pass == 0) {
-        k_mesh_narrowphase<0><<<device_sm_count() * 4, 64, 0, s>>>(w, items);
+        k_mesh_narrowphase<0><<<device_sm_count() * 8, 64, 0, s>>>(w, items);
     } else {
-        k_mesh_narrowphase<1><<<device_sm_count() * 4, 64, 0, s>>>(w, items);
+        k_mesh_narrowphase<1><<<device_sm_count() * 8, 64, 0, s>>>(w, items);
         if (w.mesh_big) k_mesh_big<<<MESH_BIG_THREADS / 64, 64, 0, s>>>(w, items);
     }
 }
@@ -3626,7 +3629,8 @@ __global__ void __launch_bounds__(128) k_ccd_find(DevWorld w, const int2 *node_w
     const int nr = w.ctr->num_ccd;
     const int n = w.n;
     const HullView hv = hull_view(w);
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(nr);
+    for (int r = spread.first; r < nr; r += spread.step) {
         CcdRec &c = w.ccd[r];
         const int a = c.body;
         const uint32_t fa = w.flags[a];
@@ -3756,7 +3760,7 @@ __global__ void __launch_bounds__(128) k_ccd_find(DevWorld w, const int2 *node_w
 }
 
 void launch_ccd_find(DevWorld &w, float dt, cudaStream_t s) {
-    k_ccd_find<<<grid_for(w.n, 128, 16), 128, 0, s>>>(w, w.node_world, dt);
+    k_ccd_find<<<spread_grid(w.n), SPREAD_BLOCK, 0, s>>>(w, w.node_world, dt);
 }
 
 // ---------------------------------------------------------------------------
@@ -4007,7 +4011,8 @@ __global__ void __launch_bounds__(128) k_cast_rays(DevWorld w, const int2 *node_
     const int n = w.n;
     const HullView hv = hull_view(w);
     const float INITIAL = 1.f + 1e-4f;  // INITIAL_EARLY_OUT_FRACTION cast-utils.ts:3
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nr; k += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(nr);
+    for (int k = spread.first; k < nr; k += spread.step) {
         const int r = order ? order[k] : k;
         const DevRay ry = rays[r];
         const float3 o = f3(ry.origin[0], ry.origin[1], ry.origin[2]);
@@ -4281,7 +4286,8 @@ __global__ void __launch_bounds__(128) k_collide_points(DevWorld w, const int2 *
                                                         DevRayFilter flt, float tol, int4 *out) {
     const int n = w.n;
     const HullView hv = hull_view(w);
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < np; r += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(np);
+    for (int r = spread.first; r < np; r += spread.step) {
         const float4 q = pts[r];
         const float3 p = xyz(q);
         const int wr = __float_as_int(q.w);
@@ -4329,7 +4335,8 @@ __global__ void __launch_bounds__(128) k_collide_points(DevWorld w, const int2 *
 void launch_collide_points(DevWorld &w, const float4 *pts, int np, const DevRayFilter &f, float tol, int4 *out,
                            cudaStream_t s) {
     if (np <= 0) return;
-    k_collide_points<<<grid_for(np, 128, 16), 128, 0, s>>>(w, w.node_world, pts, np, f, tol, out);
+    const bool few = np <= 32 * spread_grid(np);
+    k_collide_points<<<few ? spread_grid(np) : grid_for(np, 128, 16), few ? SPREAD_BLOCK : 128, 0, s>>>(w, w.node_world, pts, np, f, tol, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -4345,14 +4352,14 @@ void launch_collide_points(DevWorld &w, const float4 *pts, int np, const DevRayF
 // bodies from PASS 1's hits, as the ray queries do.  MODE picks the collector of
 // cast-shape-vs-shape.ts:165-226 as for the rays: the closest hit, the first hit found, or every
 // hit (one per convex body, one per mesh triangle) appended to hits[k * cap ...].
-constexpr int CAST_BLOCK = 32;  // one warp a block: a batch's few hundred warps spread over all SMs
 template <int PASS, int MODE>
-__global__ void __launch_bounds__(CAST_BLOCK, 16) k_cast_shapes(DevWorld w, const int2 *node_world, const DevShapeCast *qs,
+__global__ void __launch_bounds__(SPREAD_BLOCK, 16) k_cast_shapes(DevWorld w, const int2 *node_world, const DevShapeCast *qs,
                                                      int nq, DevRayFilter flt, DevShapeCastHit *hits, int cap,
                                                      int *counts) {
     const int n = w.n;
     const HullView hv = hull_view(w);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nq; k += gridDim.x * blockDim.x) {
+    const Spread spread = spread_items(nq);
+    for (int k = spread.first; k < nq; k += spread.step) {
         const DevShapeCast q = qs[k];
         const int shape = q.shape_type;
         const float4 sa = make_float4(q.params[0], q.params[1], q.params[2], q.params[3]);
@@ -4959,10 +4966,10 @@ template <int MODE>
 static void cast_shapes_mode(DevWorld &w, const DevShapeCast *qs, int nq, const DevRayFilter &f, DevShapeCastHit *hits,
                              int cap, int *counts, cudaStream_t s) {
     if (w.num_mesh_bodies > 0) {
-        k_cast_shapes<1, MODE><<<grid_for(nq, CAST_BLOCK, 64), CAST_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
-        k_cast_shapes<2, MODE><<<grid_for(nq, CAST_BLOCK, 64), CAST_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
+        k_cast_shapes<1, MODE><<<spread_grid(nq), SPREAD_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
+        k_cast_shapes<2, MODE><<<spread_grid(nq), SPREAD_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
     } else {
-        k_cast_shapes<0, MODE><<<grid_for(nq, CAST_BLOCK, 64), CAST_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
+        k_cast_shapes<0, MODE><<<spread_grid(nq), SPREAD_BLOCK, 0, s>>>(w, w.node_world, qs, nq, f, hits, cap, counts);
     }
 }
 void launch_cast_shapes(DevWorld &w, const DevShapeCast *qs, int nq, const DevRayFilter &f, DevShapeCastHit *hits,
@@ -4981,14 +4988,14 @@ void launch_cast_shapes(DevWorld &w, const DevShapeCast *qs, int nq, const DevRa
 template <int MODE>
 static void cast_rays_mode(DevWorld &w, const DevRay *rays, const int *order, int nr, const DevRayFilter &f,
                            DevRayHit *hits, int cap, int *counts, cudaStream_t s) {
+    // few rays: a warp a block and as few rays a warp as cover them (256 rays: 144 -> 53 us)
+    const bool few = nr <= 32 * spread_grid(nr);
+    const int grid = few ? spread_grid(nr) : grid_for(nr, 128, 16), block = few ? SPREAD_BLOCK : 128;
     if (w.num_mesh_bodies > 0) {
-        k_cast_rays<1, MODE><<<grid_for(nr, 128, 16), 128, 0, s>>>(w, w.node_world, rays, order, nr, f, hits, cap,
-                                                                  counts);
-        k_cast_rays<2, MODE><<<grid_for(nr, 128, 16), 128, 0, s>>>(w, w.node_world, rays, order, nr, f, hits, cap,
-                                                                  counts);
+        k_cast_rays<1, MODE><<<grid, block, 0, s>>>(w, w.node_world, rays, order, nr, f, hits, cap, counts);
+        k_cast_rays<2, MODE><<<grid, block, 0, s>>>(w, w.node_world, rays, order, nr, f, hits, cap, counts);
     } else {
-        k_cast_rays<0, MODE><<<grid_for(nr, 128, 16), 128, 0, s>>>(w, w.node_world, rays, order, nr, f, hits, cap,
-                                                                  counts);
+        k_cast_rays<0, MODE><<<grid, block, 0, s>>>(w, w.node_world, rays, order, nr, f, hits, cap, counts);
     }
 }
 void launch_cast_rays(DevWorld &w, const DevRay *rays, const int *order, int nr, const DevRayFilter &f,
