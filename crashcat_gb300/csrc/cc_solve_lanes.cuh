@@ -139,19 +139,22 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_solve_lanes(DevWorld w, CacheTab
         }
         const int n = hd.z, bits = side_bits(n, fa, fb);
         // One turn-taking pass of `visits` visits per contact: visit(v) solves the lane's contact.
-        // Every round at least one waiting contact has its turn, so the rounds are bounded.
+        // Every round at least one waiting contact has its turn, so the rounds are bounded.  All lanes
+        // read the turns before any lane visits, with a barrier of the warp between: a body passes from
+        // one visit to the next, its turn and its state, over a barrier only.
         auto turns = [&](int visits, auto &&visit) {
             int v = 0, turnA = posA, turnB = posB;
-            volatile int *turn = S.turn;
             const int most = __reduce_max_sync(FULL, has ? visits : 0) * 32;
             for (int round = 0; round < most; round++) {
                 const bool wait = has && v < visits;
                 if (!__any_sync(FULL, wait)) break;
-                if (wait && (!dynA || turn[la] == turnA) && (!dynB || turn[lb] == turnB)) {
+                const bool ready = wait && (!dynA || S.turn[la] == turnA) && (!dynB || S.turn[lb] == turnB);
+                __syncwarp();
+                if (ready) {
                     visit(v);
                     v++;
-                    if (dynA) turn[la]++;
-                    if (dynB) turn[lb]++;
+                    if (dynA) S.turn[la]++;
+                    if (dynB) S.turn[lb]++;
                     turnA += degA;
                     turnB += degB;
                 }

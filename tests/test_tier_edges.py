@@ -1,0 +1,46 @@
+"""The island tiers, queries and bounds off the sizes that the other tests meet: where a rule hands a
+call from one kernel to another, and inputs at the ends of what the entry points take.
+
+Tolerances: islands on lanes against one thread 1e-6 over three steps, as the other tests of the tiers.
+"""
+import numpy as np
+import pytest
+
+from crashcat_gb300 import _lib, scenes, world
+
+pytestmark = pytest.mark.gpu
+
+
+def make(sc, **settings):
+    ws = world.standard_settings(**settings)
+    ws.num_worlds = sc.num_worlds
+    g = world.GpuWorld(ws, sc.n + 16)
+    for p in sc.hull_points or ():
+        g.add_convex_hull(p)
+    if sc.mesh is not None:
+        g.add_triangle_mesh(*sc.mesh)
+    g.add_bodies(sc.bodies)
+    return g
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 31])
+def test_lane_islands_that_hand_one_body_on(gpu_lib, n, monkeypatch):
+    """n boxes on a slab: every contact's visit waits for the one before it on the slab, up to a
+    full warp of them."""
+    b = scenes.blank_bodies(n + 2)
+    scenes.static_floor(b, 0)
+    k = np.arange(n)
+    scenes.set_box(b, 1 + k, (0.2, 0.2, 0.2))
+    b["position"][1 + k] = np.stack([(k % 6 - 2.5) * 0.6, np.full(n, 0.5 + 0.2 - 0.005), (k // 6 - 2.5) * 0.6], 1)
+    b["linear_velocity"][1 + k] = np.random.default_rng(n).normal(scale=0.3, size=(n, 3))
+    scenes.set_box(b, n + 1, (2.0, 0.25, 2.0))
+    b["position"][n + 1] = (0.0, 0.25 - 0.005, 0.0)
+    sc = scenes.Scene("slab", b, dt=1.0 / 60.0, steps=1)
+    g = make(sc)
+    monkeypatch.setenv("CRASHCAT_SMALL_ISLAND_MAX", "64")  # past the size buckets: one thread each
+    ref = make(sc)
+    for _ in range(3):
+        g.step(sc.dt, 1)
+        ref.step(sc.dt, 1)
+        assert g.stats()["max_island_constraints"] == n + 1
+    np.testing.assert_allclose(g.get_state()[0], ref.get_state()[0], atol=1e-6)
