@@ -87,7 +87,7 @@ struct DevCounters {
     int bar_error;                      // a bounded grid-barrier wait gave up
     int giant_left[2], giant_any[2], giant_sleep;
     int giant_colours;  // most colours of a giant island this step
-    int num_small_joint_islands, num_large_joint_islands;  // islands with joints per tier
+    int num_small_joint_islands, num_coloured_islands;  // islands of k_solve_small<true> / k_solve_large
     int num_ccd;       // bodies that took the continuous-collision path this step
     int num_ccd_hits;  // of them, those whose cast hit a body
     int num_mesh_pairs;   // broadphase pairs with a triangle mesh body
@@ -545,7 +545,7 @@ struct DevWorld {
     int skip_joint_pairs;              // broadphase skips body pairs that share an enabled joint
     int *joint_partners;               // JOINT_PARTNERS per body: other bodies joined to it (-1: none)
     int *island_joint_count, *island_joint_off, *island_fill_j;
-    int *small_joint_list, *large_joint_list;  // islands with joints of the per-thread / per-CTA tiers
+    int *small_joint_list, *coloured_list;  // islands of k_solve_small<true> / k_solve_large
     // 5 x max_joints: as scattered | by (type, index) | by (priority, index, type) | colour of
     // each ranked joint | ranked joints grouped by colour (per-CTA solve)
     int *island_joints;
@@ -558,9 +558,10 @@ struct DevWorld {
     float4 *hull_points, *hull_shrunk, *hull_planes;  // planes: normal xyz, constant w
     int2 *hull_faces;                                  // first vertex index, vertex count
     int *hull_vidx;
-    // giant islands (more constraints than giant_min): solved by the whole grid
+    // giant islands: solved by the whole grid (see set_giant_min for the three lines)
     int giant_min;                         // islands with joints above this many constraints
     int giant_min_contacts;                // islands of contacts above this many
+    int giant_min_bodies;                  // islands of contacts of more bodies than this
     int giant_blocks;                      // blocks of the cooperative launch (co-resident)
     int *giant_list;
     unsigned long long *giant_claim;       // 4 x cap: contact claims, two parities | joint claims, two parities

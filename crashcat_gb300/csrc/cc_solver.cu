@@ -555,7 +555,8 @@ __device__ __forceinline__ int bucketed_island(const int *list, size_t cap, cons
 }
 
 // Island classes of k_island_classify: a per-thread or per-warp size bucket, or one of these.
-enum : int { CL_NONE = -1, CL_MID0 = 100, CL_GIANT = 1000, CL_SMALL_JOINT, CL_LARGE_JOINT, CL_LARGE, CL_BLOCK };
+// CL_COLOURED: k_solve_large takes islands of any size, with joints or without.
+enum : int { CL_NONE = -1, CL_MID0 = 100, CL_GIANT = 1000, CL_SMALL_JOINT, CL_COLOURED, CL_LARGE, CL_BLOCK };
 
 __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) {
     const int ni = w.ctr->num_islands;
@@ -570,7 +571,7 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
             const int nc = w.island_cons_count[i], nb = w.island_body_count[i];
             const int nj = joint_total(w) > 0 ? w.island_joint_count[i] : 0;
             tot = nc + nj;
-            if (nj > 0 ? nc + nj > w.giant_min : nc > w.giant_min_contacts || nb > BLOCK_L_BODIES) {
+            if (nj > 0 ? nc + nj > w.giant_min : nc > w.giant_min_contacts || nb > w.giant_min_bodies) {
                 // a pile: the whole grid solves it
                 cls = CL_GIANT;
             } else if (nj > 0) {
@@ -579,7 +580,7 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
                 cls = (nj <= c_settings.small_island_max_joints && nc <= SMALL_ISLAND_MAX_CONS &&
                        nb <= SMALL_ISLAND_MAX_BODIES)
                           ? CL_SMALL_JOINT
-                          : CL_LARGE_JOINT;
+                          : CL_COLOURED;
             } else if (nc <= c_settings.small_island_max_cons && nb <= SMALL_ISLAND_MAX_BODIES) {
                 cls = min(nc, SMALL_BUCKETS - 1);
             } else if (nc <= WARP_MAX_CONS && nb <= WARP_MAX_BODIES) {
@@ -587,8 +588,10 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
                 int b = min(max(mid_size_class(nc), 0), MID_BUCKETS - 1);
                 if (b < 2 && nb > WARP_S_BODIES) b = 2;
                 cls = CL_MID0 + b;
+            } else if (nc <= BLOCK_S_CONS && nb <= BLOCK_S_BODIES) {
+                cls = CL_LARGE;
             } else {
-                cls = nc <= BLOCK_S_CONS && nb <= BLOCK_S_BODIES ? CL_LARGE : CL_BLOCK;
+                cls = nc <= BLOCK_L_CONS && nb <= BLOCK_L_BODIES ? CL_BLOCK : CL_COLOURED;
             }
         }
         const int mx = __reduce_max_sync(FULL, tot);
@@ -602,9 +605,9 @@ __global__ void k_island_classify(DevWorld w, int *small_list, int *large_list) 
         } else if (cls == CL_SMALL_JOINT) {
             ctr = &w.ctr->num_small_joint_islands;
             list = w.small_joint_list;
-        } else if (cls == CL_LARGE_JOINT) {
-            ctr = &w.ctr->num_large_joint_islands;
-            list = w.large_joint_list;
+        } else if (cls == CL_COLOURED) {
+            ctr = &w.ctr->num_coloured_islands;
+            list = w.coloured_list;
         } else if (cls == CL_LARGE) {
             ctr = &w.ctr->num_large_islands;
             list = large_list;
@@ -1090,8 +1093,9 @@ __global__ void __launch_bounds__(128) k_solve_small(DevWorld w, CacheTables ct,
 #include "cc_solve_lanes.cuh"
 
 // ---------------------------------------------------------------------------
-// large islands with joints: one CTA per island, contacts sorted by the reference key,
-// greedily coloured in that order and swept colour by colour
+// large islands with joints, and islands of contacts past the per-CTA tier that do not go to the
+// whole grid: one CTA per island, contacts sorted by the reference key, greedily coloured in that
+// order and swept colour by colour
 // ---------------------------------------------------------------------------
 constexpr int LARGE_BLOCK = 256;
 constexpr int JOINT_COLOURS = 64;  // joint colours of the per-CTA solve; the rest go to one thread
@@ -1105,7 +1109,7 @@ __global__ void __launch_bounds__(LARGE_BLOCK) k_solve_large(DevWorld w, CacheTa
     __shared__ int s_ncol;
     __shared__ int s_colour_start[257];
     __shared__ int s_jstart[JOINT_COLOURS + 2];
-    int nl = w.ctr->num_large_joint_islands;
+    int nl = w.ctr->num_coloured_islands;
     CacheRecord *crecs = ct.recs[*ct.parity];
     for (int li = blockIdx.x; li < nl; li += gridDim.x) {
         int isl = large_list[li];
@@ -1131,7 +1135,7 @@ __global__ void __launch_bounds__(LARGE_BLOCK) k_solve_large(DevWorld w, CacheTa
             for (int k = threadIdx.x; k < nb; k += blockDim.x) prepare_body(w, bl[k]);
         // the island's joints in index order (warm start) and in (priority, index) order
         // (sortConstraintIds constraints.ts:248-261)
-        int nj = w.island_joint_count[isl];
+        int nj = joint_total(w) > 0 ? w.island_joint_count[isl] : 0;
         const int *jl = w.island_joints + (nj > 0 ? w.island_joint_off[isl] : 0);
         int *j_idx = const_cast<int *>(jl) + w.max_joints;
         int *j_pri = j_idx + w.max_joints;
@@ -2156,9 +2160,11 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
             w, ct, w.large_list + w.cap - 1, -1, &w.ctr->num_block_islands, dt, ratio, phase);
         cudaEventRecord(w.ev_join4, w.aux4_stream);
     }
-    if (joints)
+    // islands of contacts past the per-CTA tier's size come here only when giant_min was set above it
+    const bool past_block = w.max_manifolds > BLOCK_L_CONS || w.n > BLOCK_L_BODIES;
+    if (joints || (past_block && w.giant_min_bodies > BLOCK_L_BODIES))
         k_solve_large<<<device_sm_count() * 2, LARGE_BLOCK, 0, w.aux_stream>>>(
-            w, ct, w.large_joint_list, w.scratch_order, w.scratch_colour, w.scratch_claim, dt, ratio, phase);
+            w, ct, w.coloured_list, w.scratch_order, w.scratch_colour, w.scratch_claim, dt, ratio, phase);
     cudaEventRecord(w.ev_join, w.aux_stream);
     // the per-warp tier's large instance on a fourth stream, its small instance on the step's
     cudaStreamWaitEvent(w.aux3_stream, w.ev_fork, 0);
@@ -2175,7 +2181,7 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
     // giant islands: a cooperative launch (all blocks co-resident), after the other tiers so that
     // it runs alone; it returns at once when the step has no giant island, and is left out (9 us)
     // where the world is too small for one
-    const bool giant_possible = w.max_manifolds > w.giant_min_contacts || w.n > BLOCK_L_BODIES ||
+    const bool giant_possible = w.max_manifolds > w.giant_min_contacts || w.n > w.giant_min_bodies ||
                                 (nj > 0 && w.max_manifolds + nj > w.giant_min);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)w.giant_blocks);

@@ -125,15 +125,18 @@ static void drop_graph(cc_world *W) {
     }
 }
 
-// Islands with joints go to the whole grid above the given number of constraints.  So do islands of
-// contacts when the threshold is set; at its default the per-CTA tier keeps them up to its capacity
-// (a 16 x 16 x 16 heap of 11,776 contacts: 1.9 ms on one CTA, 17.5 ms on the grid, whose every
-// colour costs two grid-wide memory round trips).
+// Which islands go to the whole grid.  v > 0: those of more constraints than v; up to there one CTA
+// solves them, by k_solve_block as far as it reaches and by k_solve_large past that.  v = 0, the
+// default: islands with joints above GIANT_MIN_DEFAULT constraints, and islands of contacts past the
+// reach of k_solve_block (a 16 x 16 x 16 heap of 11,776 contacts: a step of 5.1 ms, 18.6 ms on the
+// grid, whose every colour costs two grid-wide memory round trips).
 constexpr int GIANT_MIN_DEFAULT = 8192;
 static void set_giant_min(DevWorld &w, int v) {
-    w.giant_min = v;
-    w.giant_min_contacts = v == GIANT_MIN_DEFAULT || v > BLOCK_L_CONS ? BLOCK_L_CONS : v;
+    w.giant_min = v > 0 ? v : GIANT_MIN_DEFAULT;
+    w.giant_min_contacts = v > 0 ? v : BLOCK_L_CONS;
+    w.giant_min_bodies = v > 0 ? 0x7fffffff : BLOCK_L_BODIES;
 }
+static int giant_min_set(const DevWorld &w) { return w.giant_min_bodies == BLOCK_L_BODIES ? 0 : w.giant_min; }
 
 // continuous-collision buffers, made when the first LINEAR_CAST body arrives
 static int ensure_ccd_buffers(cc_world *W) {
@@ -520,12 +523,13 @@ int cc_world_create(const cc_world_settings *s, cc_world **out) {
     ALLOC(contact_event, w.max_manifolds);
     ALLOC(removed_keys, w.max_manifolds);
     ALLOC(body_local, cap);
+    ALLOC(coloured_list, cap);
     ALLOC(giant_list, cap);
     ALLOC(giant_claim, 4 * (size_t)cap);
     ALLOC(giant_count, 4 * (GIANT_COLOURS + 2));
 #undef ALLOC
     // islands with more constraints than this are solved by the whole grid (launch-shape tunable)
-    set_giant_min(w, GIANT_MIN_DEFAULT);
+    set_giant_min(w, 0);
     if (const char *e = getenv("CRASHCAT_GIANT_MIN")) {
         int v = atoi(e);
         if (v >= 1) set_giant_min(w, v);
@@ -535,7 +539,7 @@ int cc_world_create(const cc_world_settings *s, cc_world **out) {
         int v = atoi(e);
         if (v >= 1 && v < w.giant_blocks) w.giant_blocks = v;
     }
-    if (w.giant_blocks <= 0) set_giant_min(w, 0x7fffffff);
+    if (w.giant_blocks <= 0) set_giant_min(w, 0x7fffffff);  // no grid to send them to
     if ((r = cuda_ok(cudaStreamCreateWithFlags(&W->stream, cudaStreamNonBlocking))) != CC_OK ||
         (r = cuda_ok(cudaStreamCreateWithFlags(&w.aux_stream, cudaStreamNonBlocking))) != CC_OK ||
         (r = cuda_ok(cudaStreamCreateWithFlags(&w.aux2_stream, cudaStreamNonBlocking))) != CC_OK ||
@@ -580,7 +584,7 @@ int cc_world_destroy(cc_world *W) {
                     w.scratch_colour, w.scratch_claim, w.mid_list, w.body_local, w.contact_event,
                     w.removed_keys, W->d_state_rows, w.hinges, w.island_joints, w.island_joint_count,
                     w.island_joint_off, w.island_fill_j, w.joint_wake, w.joint_partners, w.swings, w.others, w.sixdofs, w.frames,
-                    w.giant_list, w.giant_claim, w.giant_count, w.small_joint_list, w.large_joint_list,
+                    w.giant_list, w.giant_claim, w.giant_count, w.small_joint_list, w.coloured_list,
                     w.hulls, w.hull_points, w.hull_shrunk,
                     w.hull_planes, w.hull_faces, w.hull_vidx, w.ccd_flag, w.ccd_slot, w.ccd_index, w.ccd,
                     w.ccd_world_off, w.ccd_world_fill, w.ccd_seg, w.ccd_lambda, w.ccd_scan_tmp,
@@ -2023,7 +2027,7 @@ struct TuneShape {
 static TuneShape tune_shape_of(const cc_world *W) {
     const DevWorld &w = W->w;
     return TuneShape{w.epa_threads / 64 / device_sm_count(), w.epa_fetch_warp, w.warp_blocks_per_sm,
-                     W->dev_settings.small_island_max_cons, w.giant_min};
+                     W->dev_settings.small_island_max_cons, giant_min_set(w)};
 }
 static int tune_apply(cc_world *W, const TuneShape &t) {
     DevWorld &w = W->w;
@@ -2136,7 +2140,7 @@ extern "C" int cc_world_autotune(cc_world *W, float dt, int32_t steps, cc_tune_r
         if (dim == 1) cand = {1, 0};
         if (dim == 2) cand = {1, 2, 3, 4};
         if (dim == 3) cand = {4, 8, 16};
-        if (dim == 4 && piles) cand = {2048, 8192, 32768};
+        if (dim == 4 && piles && w.giant_blocks > 0) cand = {2048, 8192, 32768};
         for (int v : cand) {
             TuneShape t = cur;
             int *field = dim == 0 ? &t.epa_blocks_per_sm
@@ -2166,7 +2170,8 @@ extern "C" int cc_world_autotune(cc_world *W, float dt, int32_t steps, cc_tune_r
     rep->epa_lockstep = cur.epa_lockstep;
     rep->warp_blocks_per_sm = cur.warp_blocks_per_sm;
     rep->small_island_max_contacts = cur.small_max;
-    rep->giant_min = cur.giant_min;
+    const bool joints = w.num_hinges + w.num_swings + w.num_others + w.num_sixdofs > 0;
+    rep->giant_min = joints ? w.giant_min : w.giant_min_contacts;
     // kernel nodes of the step graph with the chosen shapes (captured by one more trial step)
     float ms = 0.f;
     if (int r = trial(ms)) return r;
@@ -2280,7 +2285,7 @@ static int ensure_joint_capacity(cc_world *W, int need_hinges, int need_swings, 
     if (!w.island_joint_count) {
         if ((r = dalloc(&w.island_joint_count, w.cap)) != CC_OK || (r = dalloc(&w.island_joint_off, w.cap)) != CC_OK ||
             (r = dalloc(&w.island_fill_j, w.cap)) != CC_OK || (r = dalloc(&w.joint_wake, 1)) != CC_OK ||
-            (r = dalloc(&w.small_joint_list, w.cap)) != CC_OK || (r = dalloc(&w.large_joint_list, w.cap)) != CC_OK ||
+            (r = dalloc(&w.small_joint_list, w.cap)) != CC_OK ||
             (r = dalloc(&w.joint_partners, (size_t)w.cap * JOINT_PARTNERS)) != CC_OK)
             return r;
         CC_TRY(cudaMemset(w.joint_partners, 0xff, sizeof(int) * (size_t)w.cap * JOINT_PARTNERS));

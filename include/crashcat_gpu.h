@@ -674,7 +674,8 @@ typedef struct cc_tune_report {
     int32_t epa_lockstep;        /* 1: a warp runs its 32 EPA items in lock-step rounds */
     int32_t warp_blocks_per_sm;  /* blocks of the per-warp island tier per SM */
     int32_t small_island_max_contacts;  /* islands up to this many contacts: one thread */
-    int32_t giant_min;           /* islands with more constraints: the whole grid */
+    int32_t giant_min;           /* islands with more constraints: the whole grid (in a world with
+                                  * joints: islands with joints) */
     int32_t graph_kernels_per_step;  /* kernel nodes of the captured step graph */
 } cc_tune_report;
 

@@ -1,7 +1,8 @@
 """The island tiers, queries and bounds off the sizes that the other tests meet: where a rule hands a
 call from one kernel to another, and inputs at the ends of what the entry points take.
 
-Tolerances: islands on lanes against one thread 1e-6 over three steps, as the other tests of the tiers.
+Tolerances: islands on lanes against one thread 1e-6 over three steps, as the other tests of the tiers; piles on one tier against another after
+one step 1e-5 m/s and, up to 92 m tall, 2e-5 m (a position near 64-128 m is held to 4e-6 m and written twice).
 """
 import numpy as np
 import pytest
@@ -44,3 +45,23 @@ def test_lane_islands_that_hand_one_body_on(gpu_lib, n, monkeypatch):
         ref.step(sc.dt, 1)
         assert g.stats()["max_island_constraints"] == n + 1
     np.testing.assert_allclose(g.get_state()[0], ref.get_state()[0], atol=1e-6)
+
+
+@pytest.mark.parametrize("base,threshold,grid", [  # 8,855 and 12,650 contacts
+    (77, None, 0), (77, "8192", 1),  # the default keeps islands of contacts on a CTA past 8,192
+    (92, None, 1), (92, "20000", 0), (92, "2147483647", 0),  # a set threshold holds past the CTA tier's reach
+])
+def test_islands_above_and_below_the_grid_threshold(gpu_lib, base, threshold, grid, monkeypatch):
+    sc = scenes.box_pyramid(base)
+    scenes.static_floor(sc.bodies, 0, half=(120.0, 0.5, 30.0), friction=0.5)
+    if threshold:
+        monkeypatch.setenv("CRASHCAT_GIANT_MIN", threshold)
+    g = make(sc, velocity_iterations=2)
+    monkeypatch.setenv("CRASHCAT_GIANT_MIN", "64")
+    ref = make(sc, velocity_iterations=2)
+    g.step(sc.dt, 1)
+    ref.step(sc.dt, 1)
+    assert (g.stats()["num_giant_islands"], ref.stats()["num_giant_islands"]) == (grid, 1)
+    a, b = g.get_state()[0], ref.get_state()[0]
+    assert np.abs(a[:, 7:13] - b[:, 7:13]).max() < 1e-5
+    assert np.abs(a[:, 0:7] - b[:, 0:7]).max() < 2e-5
