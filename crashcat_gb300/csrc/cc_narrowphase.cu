@@ -3978,9 +3978,9 @@ __device__ bool ray_vs_convex(const HullView &hv, int shape, float4 sp, float3 p
     return true;
 }
 
-// Whether a ray (in the shape's frame, unit direction) can come within the cast's tolerance (1e-3)
-// of a convex shape before max_f: the shape's own box, and the ball of a sphere, both grown by 20
-// times that and by the rounding of the frame change.  Half of the bodies whose world box a ray
+// Whether a ray (in the shape's frame, a direction of any length) can come within the cast's tolerance
+// (1e-3) of a convex shape before max_f: the shape's own box, and the ball of a sphere, both grown by
+// 20 times that and by the rounding of the frame change.  Half of the bodies whose world box a ray
 // enters fail it, and a GJK cast that misses takes as many divergent rounds as one that hits.
 __device__ __forceinline__ bool ray_near_convex(const HullView &hv, int shape, float4 sp, float3 lo, float3 ld, float len,
                                                 float max_f) {
@@ -3996,10 +3996,11 @@ __device__ __forceinline__ bool ray_near_convex(const HullView &hv, int shape, f
                                        : f3(sp.x, sp.x, sp.x);
         bl = -bh;
     }
-    const float m = 2e-2f + 1e-5f * (len + fabsf(lo.x) + fabsf(lo.y) + fabsf(lo.z));
-    if (shape == SHAPE_SPHERE && lensq3(cross3(lo, ld)) > (sp.x + m) * (sp.x + m)) return false;
+    const float d = sqrtf(lensq3(ld));
+    const float m = 2e-2f + 1e-5f * (len * d + fabsf(lo.x) + fabsf(lo.y) + fabsf(lo.z));
+    if (shape == SHAPE_SPHERE && lensq3(cross3(lo, ld)) > (sp.x + m) * (sp.x + m) * (d * d)) return false;
     const float t = ray_box_entry(lo, ld, len, bl - f3(m, m, m), bh + f3(m, m, m));
-    return t <= max_f * len + m;
+    return !(t * d > max_f * len * d + m);
 }
 
 // castRayVsShape for one body (castRayVsConvex convex.ts:54-126 with the INCLUDE_CONVEX_RADIUS

@@ -2,7 +2,7 @@
 call from one kernel to another, and inputs at the ends of what the entry points take.
 
 Tolerances: islands on lanes against one thread 1e-6 over three steps, as the other tests of the tiers; piles on one tier against another after
-one step 1e-5 m/s and, up to 92 m tall, 2e-5 m (a position near 64-128 m is held to 4e-6 m and written twice).
+one step 1e-5 m/s and, up to 92 m tall, 2e-5 m (a position near 64-128 m is held to 4e-6 m and written twice); a ray's fraction 1e-4 of 40 m (the cast's tolerance is 1 mm).
 """
 import numpy as np
 import pytest
@@ -65,3 +65,29 @@ def test_islands_above_and_below_the_grid_threshold(gpu_lib, base, threshold, gr
     a, b = g.get_state()[0], ref.get_state()[0]
     assert np.abs(a[:, 7:13] - b[:, 7:13]).max() < 1e-5
     assert np.abs(a[:, 0:7] - b[:, 0:7]).max() < 2e-5
+
+
+@pytest.mark.parametrize("length", [0.25, 1.0, 2.0, 10.0])
+def test_rays_with_a_direction_of_any_length(gpu_lib, length):
+    """A ray reaches length x direction, whatever the direction's length: the same hits as along the
+    unit direction."""
+    b = scenes.blank_bodies(4)
+    scenes.set_sphere(b, 0, 1.0)
+    scenes.set_box(b, 1, (1.0, 1.0, 1.0))
+    scenes.set_capsule(b, 2, 1.0, 0.5)
+    scenes.set_cylinder(b, 3, 0.5, 1.0)
+    y = 10.0 * np.arange(4)[:, None]
+    b["position"][:, 1] = y[:, 0]
+    b["motion_type"] = _lib.STATIC
+    b["object_layer"] = scenes.LAYER_NOT_MOVING
+    g = make(scenes.Scene("shapes", b, dt=1.0 / 60.0, steps=1))
+    x = np.array([0.0, 0.5, 0.9, 1.1, 3.0])
+    rays = np.zeros((4, 5, 7))
+    rays[..., 0], rays[..., 1], rays[..., 2] = x, y, -20.0
+    hits = []
+    for d in (1.0, length):
+        rays[..., 5], rays[..., 6] = d, 40.0 / d
+        hits.append(g.cast_rays(rays.reshape(-1, 7)))
+    assert (hits[0]["body"].reshape(4, 5) == np.where(x < 1, np.arange(4)[:, None], -1)).all()
+    np.testing.assert_array_equal(hits[1]["body"], hits[0]["body"])
+    np.testing.assert_allclose(hits[1]["fraction"], hits[0]["fraction"], atol=1e-4)
