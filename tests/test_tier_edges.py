@@ -91,3 +91,30 @@ def test_rays_with_a_direction_of_any_length(gpu_lib, length):
     assert (hits[0]["body"].reshape(4, 5) == np.where(x < 1, np.arange(4)[:, None], -1)).all()
     np.testing.assert_array_equal(hits[1]["body"], hits[0]["body"])
     np.testing.assert_allclose(hits[1]["fraction"], hits[0]["fraction"], atol=1e-4)
+
+
+def quad():
+    """A static 10 m square of two triangles at y = 0, facing up."""
+    b = scenes.blank_bodies(1)
+    b["shape_type"][0] = _lib.SHAPE_TRIANGLE_MESH
+    b["motion_type"][0] = _lib.STATIC
+    b["object_layer"][0] = scenes.LAYER_NOT_MOVING
+    sc = scenes.Scene("quad", b, dt=1.0 / 60.0, steps=1)
+    sc.mesh = (np.array([[-5, 0, -5], [5, 0, -5], [5, 0, 5], [-5, 0, 5]], np.float32),
+               np.array([[0, 2, 1], [0, 3, 2]], np.int32))
+    return sc
+
+
+@pytest.mark.parametrize("dy", [np.nan, np.inf, 0.0, -1.0])
+def test_sphere_casts_that_touch_at_the_start(gpu_lib, dy):
+    """A sphere that touches a mesh where it starts hits it at fraction 0, whatever it is moved by;
+    one 2.5 m above does not."""
+    g = make(quad())
+    c = np.zeros(2, _lib.SHAPE_CAST_DTYPE)
+    c["shape_type"] = _lib.SHAPE_SPHERE
+    c["shape_params"][:, 0] = 0.5
+    c["position"] = [(1.0, 0.4, 1.0), (1.0, 3.0, 1.0)]
+    c["quaternion"][:, 3] = 1.0
+    c["displacement"][:, 1] = dy
+    h = g.cast_shapes(c)
+    assert h["body"].tolist() == [0, -1] and h["fraction"][0] == 0.0
