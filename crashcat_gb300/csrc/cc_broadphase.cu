@@ -113,14 +113,15 @@ __device__ void exact_aabb(float4 p4, float4 q4, const double lo[3], const doubl
     }
 }
 
-// local bounds of the shape in FP64 (box.ts:77-84, sphere.ts, capsule.ts:84-94)
+// local bounds of the shape in FP64 (box.ts:77-84, sphere.ts, capsule.ts:84-94), lo <= hi on every
+// axis: half extents below zero are taken by their size, as the corners' extremes have them
 __device__ __forceinline__ void shape_bounds(const DevWorld &w, int i, uint32_t f, float4 sp, double lo[3],
                                              double hi[3]) {
     if (f & F_DECORATED) {  // the decorated shape's bounds (computeTransformedLocalBounds transformed.ts)
         const DevFrame &d = w.frames[i];
         for (int k = 0; k < 3; k++) {
-            lo[k] = d.lo[k];
-            hi[k] = d.hi[k];
+            lo[k] = fmin(d.lo[k], d.hi[k]);
+            hi[k] = fmax(d.lo[k], d.hi[k]);
         }
         return;
     }
@@ -147,9 +148,9 @@ __device__ __forceinline__ void shape_bounds(const DevWorld &w, int i, uint32_t 
     }
     double ex, ey, ez;
     if (s == SHAPE_BOX) {
-        ex = sp.x;
-        ey = sp.y;
-        ez = sp.z;
+        ex = fabsf(sp.x);
+        ey = fabsf(sp.y);
+        ez = fabsf(sp.z);
     } else if (s == SHAPE_CAPSULE) {
         ex = ez = sp.x;
         ey = da((double)sp.y, (double)sp.x);  // half height + radius
@@ -157,7 +158,7 @@ __device__ __forceinline__ void shape_bounds(const DevWorld &w, int i, uint32_t 
         ex = ez = sp.y;
         ey = sp.x;
     } else {
-        ex = ey = ez = sp.x;
+        ex = ey = ez = fabsf(sp.x);
     }
     lo[0] = -ex;
     lo[1] = -ey;

@@ -3990,15 +3990,15 @@ __device__ __forceinline__ bool ray_near_convex(const HullView &hv, int shape, f
         bl = xyz(h.lo);
         bh = xyz(h.hi);
     } else {
-        bh = shape == SHAPE_BOX       ? f3(sp.x, sp.y, sp.z)
+        bh = shape == SHAPE_BOX       ? f3(fabsf(sp.x), fabsf(sp.y), fabsf(sp.z))
              : shape == SHAPE_CAPSULE ? f3(sp.x, sp.y + sp.x, sp.x)
              : shape == SHAPE_CYLINDER ? f3(sp.y, sp.x, sp.y)
-                                       : f3(sp.x, sp.x, sp.x);
+                                       : f3(fabsf(sp.x), fabsf(sp.x), fabsf(sp.x));
         bl = -bh;
     }
     const float d = sqrtf(lensq3(ld));
     const float m = 2e-2f + 1e-5f * (len * d + fabsf(lo.x) + fabsf(lo.y) + fabsf(lo.z));
-    if (shape == SHAPE_SPHERE && lensq3(cross3(lo, ld)) > (sp.x + m) * (sp.x + m) * (d * d)) return false;
+    if (shape == SHAPE_SPHERE && lensq3(cross3(lo, ld)) > (bh.x + m) * (bh.x + m) * (d * d)) return false;
     const float t = ray_box_entry(lo, ld, len, bl - f3(m, m, m), bh + f3(m, m, m));
     return !(t * d > max_f * len * d + m);
 }

@@ -118,3 +118,30 @@ def test_sphere_casts_that_touch_at_the_start(gpu_lib, dy):
     c["displacement"][:, 1] = dy
     h = g.cast_shapes(c)
     assert h["body"].tolist() == [0, -1] and h["fraction"][0] == 0.0
+
+
+@pytest.mark.parametrize("turned", [False, True])
+@pytest.mark.parametrize("shape", ["empty", "empty_moved"])
+def test_bounds_of_extents_below_zero(gpu_lib, shape, turned):
+    """The world box of a body is the extremes of its corners, so half extents of either sign give the
+    same pairs."""
+    n = 40
+    pairs = []
+    for sign in (1.0, -1.0):
+        b = scenes.blank_bodies(n + 1)
+        for i in range(n):
+            scenes.set_sphere(b, i, 0.4)
+        b["position"][:n] = np.random.default_rng(3).uniform(-2, 2, (n, 3))
+        scenes.set_empty(b, n)
+        b["shape_params"][n, 0] = sign
+        if shape == "empty_moved":
+            b["shape_position"][n] = (0.5, 0.0, 0.0)
+        if turned:
+            b["quaternion"][n] = (0.0, 0.6, 0.0, 0.8)
+        b["motion_type"][n] = _lib.STATIC
+        b["object_layer"][n] = scenes.LAYER_NOT_MOVING
+        g = make(scenes.Scene("one of no surface", b, dt=1.0 / 60.0, steps=1))
+        g.step(0.0, 1)
+        pairs.append(sorted(tuple(sorted(p)) for p in g.get_pairs().tolist()))
+    assert any(n in p for p in pairs[0])
+    assert pairs[0] == pairs[1]
