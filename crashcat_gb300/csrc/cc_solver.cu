@@ -457,11 +457,19 @@ __global__ void k_uf_link(DevWorld w) {
     }
 }
 
+// Every body's root.  Each thread writes its own body's entry and no other: with path splitting here,
+// a thread that read an entry before its owner wrote the root into it stored an older ancestor over it
+// afterwards, and that body went to another island (the id that the scan holds at the ancestor), whose
+// solve then ran beside its own island's on the same contacts.
 __global__ void k_uf_roots(DevWorld w, int *root_flag) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.n; i += gridDim.x * blockDim.x) {
         bool act = active_body(w.flags[i]);
-        int r = act ? uf_find(w.uf_parent, i) : -1;
-        w.uf_parent[i] = r;
+        int r = -1;
+        if (act) {
+            r = i;
+            for (int p = __ldcg(&w.uf_parent[r]); p != r; p = __ldcg(&w.uf_parent[r])) r = p;
+        }
+        __stcg(&w.uf_parent[i], r);
         root_flag[i] = (act && r == i) ? 1 : 0;
     }
 }

@@ -6,6 +6,8 @@ one step 1e-5 m/s and, up to 92 m tall, 2e-5 m (a position near 64-128 m is held
 """
 import numpy as np
 import pytest
+from scipy.sparse import coo_matrix
+from scipy.sparse.csgraph import connected_components
 
 from crashcat_gb300 import _lib, scenes, world
 
@@ -145,3 +147,29 @@ def test_bounds_of_extents_below_zero(gpu_lib, shape, turned):
         pairs.append(sorted(tuple(sorted(p)) for p in g.get_pairs().tolist()))
     assert any(n in p for p in pairs[0])
     assert pairs[0] == pairs[1]
+
+
+@pytest.mark.parametrize("chains,length", [(1, 4000), (16, 1000), (1000, 30)])
+def test_every_body_is_in_the_island_of_its_contacts(gpu_lib, chains, length):
+    """Chains of touching spheres numbered at random, so that the links of an island race for its root:
+    bodies share an island exactly when contacts join them, in every one of 20 steps."""
+    n = chains * length
+    b = scenes.blank_bodies(n)
+    order = np.random.default_rng(length).permutation(n)
+    scenes.set_sphere(b, np.arange(n), 0.5)
+    k = np.arange(n)
+    b["position"][order] = np.stack([0.999 * (k % length), np.zeros(n), 3.0 * (k // length)], 1)
+    b["gravity_factor"] = 0.0
+    b["allow_sleeping"] = 0
+    g = make(scenes.Scene("chains", b, dt=1.0 / 60.0, steps=1), velocity_iterations=1, position_iterations=0)
+    rows = g.get_state()[0]
+    for _ in range(20):
+        g.set_state(rows)
+        g.step(1.0 / 60.0, 1)
+        island, contacts = g.debug_islands()
+        assert len(contacts) == chains * (length - 1)
+        joined = coo_matrix((np.ones(len(contacts)), (contacts[:, 0], contacts[:, 1])), shape=(n, n))
+        count, label = connected_components(joined, directed=False)
+        assert count == chains == g.stats()["num_islands"]
+        assert len(np.unique(np.stack([label, island]), axis=1).T) == count
+        np.testing.assert_array_equal(contacts[:, 2], island[contacts[:, 0]])
