@@ -13,6 +13,7 @@
 // body's AABB grown by the speculative contact distance, dbvt.ts:669 and
 // broadphase.ts:249) so the reported pair set equals the reference's.
 #include "cc_internal.cuh"
+#include "cc_per_device.h"
 #include "cc_sort_small.cuh"
 
 namespace cc {
@@ -603,12 +604,8 @@ static void launch_tree(DevWorld &w, cudaStream_t s) {
     int wbits = 0;
     while ((1 << wbits) < w.num_worlds) wbits++;
     if (n <= TREE_SMALL) {
-        static bool attr_set = false;  // set on the first (eager) step, before any graph capture
-        if (!attr_set) {
-            cudaFuncSetAttribute(k_tree_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)SmallSort::bytes(TREE_SMALL));
-            attr_set = true;
-        }
+        static PerDevice shared;
+        shared.get([] { return allow_shared(SmallSort::bytes(TREE_SMALL), k_tree_small); });
         k_tree_small<<<1, SORT_BLOCK, SmallSort::bytes(n), s>>>(w, w.scene, w.node_world, 30 + wbits);
         return;
     }

@@ -5,22 +5,21 @@
 #include <utility>
 
 #include "cc_internal.cuh"
+#include "cc_per_device.h"
 #include "cc_sort_small.cuh"
 
 namespace cc {
 
-// SM count of the current device, read once per device (a benign race: every writer stores the
-// same value); 152 when the attribute cannot be read
+// SM count of the current device; 152 when the attribute cannot be read
 int device_sm_count() {
-    constexpr int MAX_DEVICES = 64;
-    static int cached[MAX_DEVICES] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 152;
-    int v = cached[dev];
-    if (v > 0) return v;
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 152;
-    cached[dev] = v;
-    return v;
+    static PerDevice count;
+    return count.get([] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
+            v = 152;
+        return v;
+    });
 }
 
 constexpr int SCAN_BLOCK = 1024;
@@ -289,12 +288,8 @@ void radix_sort_pairs_u64(unsigned long long *keys, unsigned long long *keys_alt
                           int bits, int *tmp, cudaStream_t s, const int *) {
     if (n <= 1) return;
     if (n <= SORT_SMALL) {
-        static bool attr_set = false;
-        if (!attr_set) {
-            cudaFuncSetAttribute(k_radix_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)SmallSort::bytes(SORT_SMALL));
-            attr_set = true;
-        }
+        static PerDevice shared;
+        shared.get([] { return allow_shared(SmallSort::bytes(SORT_SMALL), k_radix_sort_small); });
         k_radix_sort_small<<<1, SORT_BLOCK, SmallSort::bytes(n), s>>>(keys, vals, n, bits);
         return;
     }

@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "cc_internal.cuh"
+#include "cc_per_device.h"
 #include "cc_swing.cuh"
 
 namespace cc {
@@ -2119,42 +2120,32 @@ void launch_solver(DevWorld &w, float dt, float ratio, cudaStream_t s, cudaEvent
         cudaEventRecord(w.ev_join2, w.aux2_stream);
     // the per-warp tier's two instances: their shared memory, and for the small one the blocks
     // that are resident at once (its first round assigns islands to every warp up front)
-    static bool warp_attr_set = false;  // set on the first (eager) step, before any graph capture
-    static int warp_s_blocks_per_sm = 1;
-    static bool warp_s_sized = false;  // sized after the carveout is first set
+    static PerDevice warp_shared, warp_s_shared, warp_s_blocks, block_shared;
     const size_t warp_smem = sizeof(WarpIsland) * WARPS_PER_BLOCK;
     const size_t warp_s_smem = sizeof(WarpIslandS) * WARPS_PER_BLOCK;
-    if (!warp_attr_set) {
-        cudaFuncSetAttribute(k_solve_warp<WarpIsland>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_smem);
-        cudaFuncSetAttribute(k_solve_warp<WarpIslandS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)warp_s_smem);
-        warp_attr_set = true;
-    }
+    warp_shared.get([&] { return allow_shared(warp_smem, k_solve_warp<WarpIsland>); });
+    warp_s_shared.get([&] { return allow_shared(warp_s_smem, k_solve_warp<WarpIslandS>); });
     if (w.warp_carveout >= 0) {
         cudaFuncSetAttribute(k_solve_warp<WarpIsland>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              w.warp_carveout);
         cudaFuncSetAttribute(k_solve_warp<WarpIslandS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              w.warp_carveout);
     }
-    if (!warp_s_sized) {
+    const int warp_s_blocks_per_sm = warp_s_blocks.get([&] {  // sized after the carveout is first set
         int nbk = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbk, k_solve_warp<WarpIslandS>, WARP_BLOCK, warp_s_smem) ==
-                cudaSuccess &&
-            nbk > 0)
-            warp_s_blocks_per_sm = nbk;
-        warp_s_sized = true;
-    }
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbk, k_solve_warp<WarpIslandS>, WARP_BLOCK, warp_s_smem) !=
+                cudaSuccess ||
+            nbk < 1)
+            nbk = 1;
+        return nbk;
+    });
     // the per-CTA and per-warp classes hold disjoint islands: run them side by side
     cudaEventRecord(w.ev_fork, s);
     cudaStreamWaitEvent(w.aux_stream, w.ev_fork, 0);
-    static bool block_attr_set = false;
-    if (!block_attr_set) {
-        cudaFuncSetAttribute(k_solve_block<BlockTierS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)BlockTierS::SMEM);
-        cudaFuncSetAttribute(k_solve_block<BlockTierL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)BlockTierL::SMEM);
-        block_attr_set = true;
-    }
+    block_shared.get([] {
+        return allow_shared(BlockTierS::SMEM, k_solve_block<BlockTierS>) &
+               allow_shared(BlockTierL::SMEM, k_solve_block<BlockTierL>);
+    });
     // no more blocks than the world can have islands of the instance's size; none at all where it
     // cannot have one
     const int sms = device_sm_count();
@@ -2483,11 +2474,8 @@ void launch_ccd(DevWorld &w, float dt, cudaStream_t s) {
                        w.ccd_scan_tmp, s);
     cudaMemsetAsync(w.ccd_world_fill, 0, sizeof(int) * (size_t)w.num_worlds, s);
     k_ccd_scatter<<<grid_for(w.n, 256), 256, 0, s>>>(w);
-    static bool attr_set = false;  // set on the first (eager) step, before any graph capture
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_ccd_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CcdSort));
-        attr_set = true;
-    }
+    static PerDevice shared;
+    shared.get([] { return allow_shared(sizeof(CcdSort), k_ccd_resolve); });
     k_ccd_resolve<<<std::min(w.num_worlds, 2 * device_sm_count()), CCD_BLOCK, sizeof(CcdSort), s>>>(w);
 }
 
