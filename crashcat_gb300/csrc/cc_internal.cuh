@@ -130,9 +130,11 @@ struct DevSettings {
     uint32_t cast_pairs[CC_MAX_LAYERS];
     int small_island_max_cons;  // islands up to this many contacts run on one thread
     int small_island_max_joints;  // islands with joints: up to this many joints run on one thread
-    unsigned wait_polls;        // polls of a bounded device wait (grid barrier) before it gives up
+    unsigned wait_polls;        // polls of a bounded device wait (the grid barrier; 32 times as many of a CTA
+                                // island's turns) before it gives up
     int link_attempts;          // attempts of one union-find link before it gives up (OVF_ISLAND)
-    int test_withhold_block;    // test hook: block 0 of the whole-grid solve skips its barriers
+    int test_withhold_block;    // test hook: block 0 of the whole-grid solve skips its barriers, warp 0 of a
+                                // CTA island's solve does not report its chunks
 };
 
 // Manifold produced by the narrowphase for one body pair (<= 4 points),

@@ -370,11 +370,13 @@ __global__ void __launch_bounds__(T::THREADS, 1)
         }
         __syncthreads();  // the lists are done with: their memory takes the state
         float *state = (float *)block_smem;  // 7 per body: velocities (6), then in the position sweeps the pose
-        // a chunk's turn: every chunk of the earlier levels is done (bounded wait)
+        // a chunk's turn: every chunk of the earlier levels is done.  The wait is bounded: 32 polls of
+        // shared memory for each poll of the whole-grid solve's barrier, which pauses between them
+        const unsigned poll_limit = min(c_settings.wait_polls, ~0u / 32) * 32;
         auto turn = [&](int want) -> bool {
             bool ok = true;
             for (unsigned polls = 0; s_done < want; polls++)
-                if (s_fail || polls > (1u << 26)) {
+                if (s_fail || polls > poll_limit) {
                     s_fail = 1;
                     atomicOr(&w.ctr->overflow, OVF_TIMEOUT);
                     ok = false;
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(T::THREADS, 1)
         };
         auto chunk_done = [&]() {
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0 && !(c_settings.test_withhold_block && wid == 0)) {
                 __threadfence_block();
                 atomicAdd((int *)&s_done, 1);
             }

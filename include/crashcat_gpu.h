@@ -129,7 +129,8 @@ typedef struct cc_world_settings {
     /* bounds of the device-side waits (no counterpart in the reference: the single-threaded step
      * never waits).  device_wait_polls: polls of a grid barrier of the whole-grid island solve
      * before it gives up, sets CC_ERR_TIMEOUT for the step and every block leaves (0: 2^21, about
-     * 0.2 s).  island_link_attempts: compare-and-swap attempts of one union-find link before it
+     * 0.2 s); the solve of one large island by one CTA waits for at most 32 times as many polls of
+     * its own, shorter ones.  island_link_attempts: compare-and-swap attempts of one union-find link before it
      * gives up; the step then skips its solve and returns CC_ERR_CAPACITY (0: 2^20). */
     int32_t device_wait_polls;
     int32_t island_link_attempts;

@@ -173,3 +173,22 @@ def test_every_body_is_in_the_island_of_its_contacts(gpu_lib, chains, length):
         assert count == chains == g.stats()["num_islands"]
         assert len(np.unique(np.stack([label, island]), axis=1).T) == count
         np.testing.assert_array_equal(contacts[:, 2], island[contacts[:, 0]])
+
+
+@pytest.mark.parametrize("base", [20, 53])  # 590 and 4,187 contacts: the CTA tier's two sizes
+def test_turn_of_a_cta_island_runs_out_with_a_status(gpu_lib, base, monkeypatch):
+    """With a warp's finished chunks not reported, the other warps' wait for their turn runs out after
+    the polls that the settings allow: the step returns CC_ERR_TIMEOUT with OVF_TIMEOUT in the counters,
+    and the device keeps answering."""
+    monkeypatch.setenv("CRASHCAT_TEST_WITHHOLD_BARRIER", "1")
+    sc = scenes.box_pyramid(base)
+    scenes.static_floor(sc.bodies, 0, half=(120.0, 0.5, 30.0), friction=0.5)
+    g = make(sc, device_wait_polls=2000)
+    with pytest.raises(_lib.CCError) as e:
+        g.step(sc.dt, 1)
+    assert e.value.status == _lib.CC_ERR_TIMEOUT
+    assert g.stats()["num_giant_islands"] == 0 and g.stats()["overflow_flags"] & 64
+    monkeypatch.delenv("CRASHCAT_TEST_WITHHOLD_BARRIER")
+    ok = make(sc)
+    assert ok.step(sc.dt, 3) == _lib.CC_OK
+    assert np.isfinite(ok.get_state()[0]).all()
