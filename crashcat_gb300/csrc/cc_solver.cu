@@ -2341,7 +2341,12 @@ __device__ void ccd_hit(DevWorld &w, CcdRec &c, CcdRec *cb, float2 &lam) {
 // global memory took 4.8 ms); the hits, a few in a hundred, follow one another on one thread.  A move
 // without a hit is seen by others only as the body that a later record hits, so it may wait
 // until such a record needs it, or until the end.  Worlds of more than CCD_SORT records take one thread.
-constexpr int CCD_SORT = 4096, CCD_BLOCK = 256;
+// So do worlds of few records when there are more worlds than CTAs at once: the CTA's two sorts and
+// its barriers cost the same for one record as for dozens, and the worlds queue for them.  The more
+// rounds of CTAs the worlds make, the more records a thread may take (a step of 4,096 worlds, 14
+// rounds, on CTAs and on threads: 1 record each 390 and 334 us, 16 763 and 648 us, 64 1,915 and 1,657
+// us; of 512 worlds, 2 rounds: 8 records 346 and 347 us, 16 417 and 428 us, 64 588 and 690 us).
+constexpr int CCD_SORT = 4096, CCD_BLOCK = 256, CCD_FEW_A_ROUND = 5, CCD_FEW_MAX = 64;
 struct CcdSort {
     unsigned long long key[CCD_SORT];
     int by_slot[CCD_SORT];     // record of each slot (body order)
@@ -2371,7 +2376,16 @@ __device__ void ccd_resolve_serial(DevWorld &w, int wd, int o0, int m) {
     }
     w.ccd_lambda[wd] = lam;
 }
-__global__ void __launch_bounds__(CCD_BLOCK) k_ccd_resolve(DevWorld w) {
+__global__ void __launch_bounds__(SPREAD_BLOCK) k_ccd_resolve_few(DevWorld w, int few) {
+    if (w.ctr->num_ccd == 0) return;
+    const Spread sp = spread_items(w.num_worlds);
+    for (int wd = sp.first; wd < w.num_worlds; wd += sp.step) {
+        const int o0 = w.ccd_world_off[wd], m = w.ccd_world_off[wd + 1] - o0;
+        if (m > 0 && m <= few) ccd_resolve_serial(w, wd, o0, m);
+    }
+}
+// few: worlds of up to so many records are k_ccd_resolve_few's
+__global__ void __launch_bounds__(CCD_BLOCK) k_ccd_resolve(DevWorld w, int few) {
     if (w.ctr->num_ccd == 0) return;
     extern __shared__ __align__(16) unsigned char ccd_smem[];
     __shared__ int s_hits;
@@ -2380,7 +2394,7 @@ __global__ void __launch_bounds__(CCD_BLOCK) k_ccd_resolve(DevWorld w) {
     const int tid = threadIdx.x, lane = tid & 31;
     for (int wd = blockIdx.x; wd < w.num_worlds; wd += gridDim.x) {
         const int o0 = w.ccd_world_off[wd], m = w.ccd_world_off[wd + 1] - o0;
-        if (m <= 0) continue;
+        if (m <= few) continue;
         if (m > CCD_SORT) {
             if (tid == 0) ccd_resolve_serial(w, wd, o0, m);
             continue;
@@ -2476,7 +2490,10 @@ void launch_ccd(DevWorld &w, float dt, cudaStream_t s) {
     k_ccd_scatter<<<grid_for(w.n, 256), 256, 0, s>>>(w);
     static PerDevice shared;
     shared.get([] { return allow_shared(sizeof(CcdSort), k_ccd_resolve); });
-    k_ccd_resolve<<<std::min(w.num_worlds, 2 * device_sm_count()), CCD_BLOCK, sizeof(CcdSort), s>>>(w);
+    const int at_once = 2 * device_sm_count(), rounds = (w.num_worlds + at_once - 1) / at_once;
+    const int few = rounds > 1 ? std::min(CCD_FEW_A_ROUND * rounds, CCD_FEW_MAX) : 0;
+    if (few > 0) k_ccd_resolve_few<<<spread_grid(w.num_worlds), SPREAD_BLOCK, 0, s>>>(w, few);
+    k_ccd_resolve<<<std::min(w.num_worlds, at_once), CCD_BLOCK, sizeof(CcdSort), s>>>(w, few);
 }
 
 // blocks of the giant-island launch: one per SM, fewer if the kernel cannot be resident at that

@@ -192,3 +192,42 @@ def test_turn_of_a_cta_island_runs_out_with_a_status(gpu_lib, base, monkeypatch)
     ok = make(sc)
     assert ok.step(sc.dt, 3) == _lib.CC_OK
     assert np.isfinite(ok.get_state()[0]).all()
+
+
+def bullet_worlds(worlds, k):
+    """`worlds` worlds, in each k swept spheres: in three, one hits a wall, one the sphere before it
+    (cast too), and one meets nothing."""
+    b = scenes.blank_bodies(2 * k)
+    i = np.arange(k)
+    scenes.set_box(b, i, (0.05, 1.0, 1.0))
+    scenes.set_sphere(b, k + i, 0.2)
+    at = np.stack([np.zeros(k), np.zeros(k), 4.0 * (i // 3)], 1)
+    b["position"][:k] = at + (5.0, 0.0, 0.0)
+    b["position"][:k][i % 3 != 0] += (0.0, 500.0, 0.0)  # no wall for these
+    b["position"][k:] = at
+    b["position"][k:][i % 3 == 1] += (-2.0, 0.1, 0.0)
+    b["position"][k:][i % 3 == 2] += (0.0, 50.0, 0.0)
+    b["motion_type"][:k] = _lib.STATIC
+    b["object_layer"][:k] = scenes.LAYER_NOT_MOVING
+    b["linear_velocity"][k:, 0] = np.where(i % 3 == 1, 450.0, 320.0) + i % 7
+    b["motion_quality"][k:] = 1
+    b["gravity_factor"][k:] = 0.0
+    out = np.tile(b, worlds)
+    out["world"] = np.repeat(np.arange(worlds), 2 * k)
+    return scenes.Scene("bullets", out, dt=1.0 / 60.0, steps=1, num_worlds=worlds)
+
+
+@pytest.mark.parametrize("k", [1, 2, 15, 16, 25])  # threads up to 15 records of 700 worlds
+def test_swept_bodies_of_many_worlds(gpu_lib, k):
+    """More worlds than CTAs at once: worlds of few records take a thread, the others a CTA.  Every
+    world ends as the same bodies do in a world handle of their own, which take a CTA."""
+    worlds = 700
+    many, one = make(bullet_worlds(worlds, k)), make(bullet_worlds(1, k))
+    for step in range(2):
+        many.step(1.0 / 60.0, 1)
+        one.step(1.0 / 60.0, 1)
+        s, t = many.stats(), one.stats()
+        assert (s["num_ccd"], s["num_ccd_hits"]) == (worlds * t["num_ccd"], worlds * t["num_ccd_hits"])
+        assert step > 0 or t["num_ccd_hits"] >= (k + 2) // 3
+    a, b = many.get_state()[0].reshape(worlds, 2 * k, -1), one.get_state()[0]
+    np.testing.assert_array_equal(a, np.broadcast_to(b, a.shape))
