@@ -2022,16 +2022,16 @@ extern "C" int cc_world_rollout_grad(cc_world *W, float dt, int32_t n_steps, int
 // launch-shape autotuner
 // ---------------------------------------------------------------------------
 struct TuneShape {
-    int epa_blocks_per_sm, epa_lockstep, warp_blocks_per_sm, small_max, giant_min;
+    int epa_blocks, epa_lockstep, warp_blocks_per_sm, small_max, giant_min;  // EPA blocks: of the whole grid
 };
 static TuneShape tune_shape_of(const cc_world *W) {
     const DevWorld &w = W->w;
-    return TuneShape{w.epa_threads / 64 / device_sm_count(), w.epa_fetch_warp, w.warp_blocks_per_sm,
+    return TuneShape{w.epa_threads / 64, w.epa_fetch_warp, w.warp_blocks_per_sm,
                      W->dev_settings.small_island_max_cons, giant_min_set(w)};
 }
 static int tune_apply(cc_world *W, const TuneShape &t) {
     DevWorld &w = W->w;
-    int blocks = t.epa_blocks_per_sm * device_sm_count();
+    const int blocks = t.epa_blocks;
     if (blocks > W->epa_packed_blocks) {
         if (w.epa_packed) cudaFree(w.epa_packed);
         w.epa_packed = nullptr;
@@ -2133,17 +2133,17 @@ extern "C" int cc_world_autotune(cc_world *W, float dt, int32_t steps, cc_tune_r
     rep->default_ms = best;
     const bool piles = W->last_ctr.max_island_constraints > 2048;
     const int sms = device_sm_count();
-    const int epa_cap = epa_max_threads() / 64 / sms;
+    const int epa_cap = epa_max_threads() / 64;
     for (int dim = 0; dim < 5; dim++) {
         std::vector<int> cand;
-        if (dim == 0) cand = {2, 4, 6, 8};
+        if (dim == 0) cand = {2 * sms, 4 * sms, 6 * sms, 8 * sms};
         if (dim == 1) cand = {1, 0};
         if (dim == 2) cand = {1, 2, 3, 4};
         if (dim == 3) cand = {4, 8, 16};
         if (dim == 4 && piles && w.giant_blocks > 0) cand = {2048, 8192, 32768};
         for (int v : cand) {
             TuneShape t = cur;
-            int *field = dim == 0 ? &t.epa_blocks_per_sm
+            int *field = dim == 0 ? &t.epa_blocks
                                   : dim == 1 ? &t.epa_lockstep
                                   : dim == 2 ? &t.warp_blocks_per_sm : dim == 3 ? &t.small_max : &t.giant_min;
             if (*field == v) continue;
@@ -2166,7 +2166,7 @@ extern "C" int cc_world_autotune(cc_world *W, float dt, int32_t steps, cc_tune_r
     W->steps_done = steps_done;
     rep->tuned_ms = best;
     rep->trials = trials;
-    rep->epa_blocks_per_sm = cur.epa_blocks_per_sm;
+    rep->epa_blocks_per_sm = cur.epa_blocks / sms;
     rep->epa_lockstep = cur.epa_lockstep;
     rep->warp_blocks_per_sm = cur.warp_blocks_per_sm;
     rep->small_island_max_contacts = cur.small_max;

@@ -671,7 +671,7 @@ typedef struct cc_tune_report {
     float default_ms;            /* ms per step with the shapes the world had */
     float tuned_ms;              /* ms per step with the shapes it keeps */
     int32_t trials;
-    int32_t epa_blocks_per_sm;   /* 64-thread EPA blocks per SM */
+    int32_t epa_blocks_per_sm;   /* 64-thread EPA blocks per SM (0: fewer blocks than SMs) */
     int32_t epa_lockstep;        /* 1: a warp runs its 32 EPA items in lock-step rounds */
     int32_t warp_blocks_per_sm;  /* blocks of the per-warp island tier per SM */
     int32_t small_island_max_contacts;  /* islands up to this many contacts: one thread */

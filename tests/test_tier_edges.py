@@ -231,3 +231,19 @@ def test_swept_bodies_of_many_worlds(gpu_lib, k):
         assert step > 0 or t["num_ccd_hits"] >= (k + 2) // 3
     a, b = many.get_state()[0].reshape(worlds, 2 * k, -1), one.get_state()[0]
     np.testing.assert_array_equal(a, np.broadcast_to(b, a.shape))
+
+
+@pytest.mark.parametrize("kind", ["falling", "stack", "pairs"])
+def test_autotune_of_a_small_world(gpu_lib, kind):
+    """A small world starts with fewer EPA blocks than SMs.  Whether or not the tuner finds a shape that
+    is faster, the world steps on, and as without the tuner."""
+    sc = {"falling": lambda: scenes.free_fall(n=8), "stack": lambda: scenes.box_stack(height=5),
+          "pairs": lambda: scenes.random_pairs_scene(n=40)}[kind]()
+    tuned, plain = make(sc), make(sc)
+    for g in (tuned, plain):
+        g.step(sc.dt, 5)
+    rep = tuned.autotune(sc.dt, 1)
+    assert rep["epa_blocks_per_sm"] >= 0 and rep["giant_min"] == 12288
+    for g in (tuned, plain):
+        assert g.step(sc.dt, 5) == _lib.CC_OK
+    np.testing.assert_allclose(tuned.get_state()[0], plain.get_state()[0], atol=1e-4)
