@@ -10,6 +10,7 @@ from scipy.sparse import coo_matrix
 from scipy.sparse.csgraph import connected_components
 
 from crashcat_gb300 import _lib, scenes, world
+from oracle import pyoracle
 
 pytestmark = pytest.mark.gpu
 
@@ -247,3 +248,231 @@ def test_autotune_of_a_small_world(gpu_lib, kind):
     for g in (tuned, plain):
         assert g.step(sc.dt, 5) == _lib.CC_OK
     np.testing.assert_allclose(tuned.get_state()[0], plain.get_state()[0], atol=1e-4)
+
+
+@pytest.mark.parametrize("extra", [0, 1])
+def test_islands_at_the_count_that_ends_the_lanes(gpu_lib, extra):
+    """Pyramids of 1, 5, 12, 22 and 35 contacts among falling boxes, 16,384 islands (contacts on lanes) or
+    one more (threads and both per-warp sizes): the pyramids end as they do alone."""
+    parts, alone = [], []
+    for base in (1, 2, 3, 4, 5):
+        sc = scenes.box_pyramid(base)
+        g = make(sc)
+        for _ in range(3):
+            g.step(sc.dt, 1)
+        alone.append(g.get_state()[0])
+        b = sc.bodies.copy()
+        b["world"] = base
+        parts.append(b)
+    lone = 16384 - len(parts) + extra
+    k = np.arange(lone)
+    b = scenes.blank_bodies(lone)
+    scenes.set_box(b, k, (0.2, 0.2, 0.2))
+    b["position"] = np.stack([2.0 * (k % 128), np.full(lone, 30.0), 2.0 * (k // 128)], 1)
+    sc = scenes.Scene("many", np.concatenate(parts + [b]), dt=1.0 / 60.0, steps=3, num_worlds=6)
+    g = make(sc)
+    for _ in range(3):
+        g.step(sc.dt, 1)
+        assert g.stats()["num_islands"] == 16384 + extra
+    rows, at = g.get_state()[0], 0
+    for a in alone:
+        np.testing.assert_allclose(rows[at:at + len(a)], a, atol=1e-6)
+        at += len(a)
+
+
+def snake(n):
+    """n spheres numbered at random, each touching the next, in rows of 63 joined at their ends: n - 1
+    contacts, no gravity."""
+    k = np.arange(n)
+    row, at = k // 64, k % 64
+    x = np.where(row % 2 == 0, np.minimum(at, 62), 62 - np.minimum(at, 62))
+    z = 2.0 * row + (at == 63)
+    rng = np.random.default_rng(n)
+    order = rng.permutation(n)
+    b = scenes.blank_bodies(n)
+    scenes.set_sphere(b, k, 0.5)
+    b["position"][order] = 0.999 * np.stack([x, np.zeros(n), z], 1)
+    b["linear_velocity"] = rng.normal(scale=0.3, size=(n, 3))
+    b["gravity_factor"] = 0.0
+    return scenes.Scene("snake", b, dt=1.0 / 60.0, steps=1)
+
+
+@pytest.mark.parametrize("n,grid", [(127, 0), (128, 0), (129, 0), (2047, 0), (2048, 0), (2049, 0), (6144, 0), (6145, 1)])
+def test_islands_at_the_body_limits(gpu_lib, n, grid, monkeypatch):
+    """The tiers' limits of bodies, with half as many contacts as they take: 128 on a warp, 2,048 and
+    6,144 on a CTA; against the grid, and the grid against one CTA."""
+    sc = snake(n)
+    g = make(sc)
+    monkeypatch.setenv("CRASHCAT_GIANT_MIN", "2147483647" if grid else "64")
+    ref = make(sc)
+    g.step(sc.dt, 1)
+    ref.step(sc.dt, 1)
+    s, t = g.stats(), ref.stats()
+    assert s["max_island_constraints"] == t["max_island_constraints"] == n - 1 and s["num_islands"] == 1
+    assert (s["num_giant_islands"], t["num_giant_islands"]) == (grid, 1 - grid)
+    a, b = g.get_state()[0], ref.get_state()[0]
+    assert np.abs(a[:, 7:13] - b[:, 7:13]).max() < 1e-5
+    assert np.abs(a[:, 0:7] - b[:, 0:7]).max() < 3e-5  # up to 192 m from the origin
+
+
+@pytest.mark.parametrize("iterations", [12, 13, 30])
+def test_position_sweeps_past_one_schedule(gpu_lib, iterations, monkeypatch):
+    sc = scenes.box_pyramid(20)
+    sc.bodies["position"][1:, 1] -= 0.02  # pressed in by more than the slop: every sweep moves something
+    g = make(sc, position_iterations=iterations)
+    monkeypatch.setenv("CRASHCAT_GIANT_MIN", "64")
+    ref = make(sc, position_iterations=iterations)
+    g.step(sc.dt, 1)
+    ref.step(sc.dt, 1)
+    a, b = g.get_state()[0], ref.get_state()[0]
+    assert np.abs(a[:, 7:13] - b[:, 7:13]).max() < 1e-5
+    assert np.abs(a[:, 0:7] - b[:, 0:7]).max() < 2e-5
+
+
+def test_cta_tiers_side_by_side(gpu_lib, monkeypatch):
+    """Islands of both sizes of the CTA tier and jointed ones of the coloured solve in one step, on their
+    streams over the shared scratch: each ends as it does in a world handle of its own."""
+    monkeypatch.setenv("CRASHCAT_SMALL_JOINTS_MAX", "0")
+
+    def build(scs):
+        b, hinges, swings, at = [], [], [], 0
+        for k, sc in enumerate(scs):
+            rows = sc.bodies.copy()
+            rows["world"] = k
+            b.append(rows)
+            for joints, of in ((hinges, sc.hinges), (swings, sc.swings)):
+                if of is not None:
+                    j = of.copy()
+                    j["body_a"] += at
+                    j["body_b"] += at
+                    joints.append(j)
+            at += len(rows)
+        ws = world.standard_settings()
+        ws.num_worlds = len(scs)
+        g = world.GpuWorld(ws, at + 16)
+        g.add_bodies(np.concatenate(b))
+        if hinges:
+            g.add_hinges(np.concatenate(hinges))
+            g.add_swing_twists(np.concatenate(swings))
+        g.set_skip_joint_pairs(True)
+        return g
+
+    big = scenes.box_pyramid(55)  # 4,510 contacts
+    scenes.static_floor(big.bodies, 0, half=(120.0, 0.5, 30.0), friction=0.5)
+    scs = [scenes.ragdolls(num=4, arena=12.0), scenes.box_pyramid(15), big, scenes.box_pyramid(20)]
+    together = build(scs)
+    for _ in range(3):
+        together.step(1.0 / 60.0, 1)
+    rows, at = together.get_state()[0], 0
+    for sc in scs:
+        g = build([sc])
+        for _ in range(3):
+            g.step(1.0 / 60.0, 1)
+        np.testing.assert_allclose(rows[at:at + sc.n], g.get_state()[0], atol=1e-6)
+        at += sc.n
+
+
+def triples(groups, extra):
+    """Groups of three swept spheres and a wall: sphere A would hit the wall half way through the step;
+    B meets A at 0.3 of it, which cancels A's hit; C meets A at 0.8, after A's turn.  `extra` more meet
+    nothing."""
+    n = 3 * groups + extra
+    b = scenes.blank_bodies(groups + n)
+    wall, s = np.arange(groups), groups + np.arange(n)
+    scenes.set_box(b, wall, (0.05, 0.8, 0.5))
+    scenes.set_sphere(b, s, 0.2)
+    b["motion_type"][wall] = _lib.STATIC
+    b["object_layer"][wall] = scenes.LAYER_NOT_MOVING
+    lane = np.stack([40.0 * (wall % 16), np.zeros(groups), 3.0 * (wall // 16)], 1)
+    b["position"][wall] = lane + (2.25, 0.0, 0.0)
+    for k, (y, vy) in enumerate(((-1.6, 240.0), (3.6, -240.0), (0.0, 0.0))):  # B, C, A
+        i = groups + 3 * wall + k
+        b["position"][i] = lane + (0.0, y, 0.0)
+        b["linear_velocity"][i] = (240.0, vy, 0.0)
+    b["position"][s[3 * groups:]] = np.stack([np.arange(extra), np.full(extra, 300.0), np.zeros(extra)], 1)
+    b["linear_velocity"][s[3 * groups:], 2] = 240.0
+    b["motion_quality"][s] = 1
+    b["gravity_factor"][s] = 0.0
+    return scenes.Scene("triples", b, dt=1.0 / 60.0, steps=1)
+
+
+@pytest.mark.parametrize("groups", [1, 11, 1365])  # 1,365: 4,096 and 4,097 records, on chip and on one thread
+def test_swept_bodies_that_hit_one_another(gpu_lib, oracle_lib, groups):
+    """A record whose hit was cancelled moves at its turn, before a later record hits it."""
+    rows = []
+    for extra in (1, 2):
+        sc = triples(groups, extra)
+        g = make(sc)
+        g.step(sc.dt, 1)
+        assert (g.stats()["num_ccd"], g.stats()["num_ccd_hits"]) == (3 * groups + extra, 3 * groups)
+        rows.append(g.get_state()[0][:4 * groups])
+    np.testing.assert_array_equal(rows[0], rows[1])
+    if groups < 100:
+        o = pyoracle.OracleWorld(world.standard_settings(), sc.bodies)
+        o.step(sc.dt, 1)
+        st = o.state()[:4 * groups]
+        np.testing.assert_allclose(rows[0][:, 0:3], st[:, 0:3], atol=5e-3)
+        np.testing.assert_allclose(rows[0][:, 7:10], st[:, 7:10], atol=5e-2)
+
+
+@pytest.mark.parametrize("offset", [0.0, 2000.0])
+def test_sphere_casts_far_from_the_origin(gpu_lib, oracle_lib, offset):
+    """Long sphere sweeps onto a terrain whose vertices lie `offset` from the mesh's origin, against the
+    oracle: as many hits, 99 % of the distances within 2e-3 m and ten times the spacing of FP32 there, all
+    within 0.1 m (as the other test of casts onto a terrain)."""
+    verts, tris = scenes.heightfield(24, 1.0, 2.0, 5)
+    b = scenes.blank_bodies(1)
+    b["shape_type"][0] = _lib.SHAPE_TRIANGLE_MESH
+    b["motion_type"][0] = _lib.STATIC
+    b["object_layer"][0] = scenes.LAYER_NOT_MOVING
+    sc = scenes.Scene("far", b, dt=1.0 / 60.0, steps=1)
+    sc.mesh = ((np.asarray(verts).reshape(-1, 3) + (offset, 0.0, -offset)).astype(np.float32), tris)
+    g = make(sc)
+    o = pyoracle.OracleWorld(world.standard_settings(), b, (), [g.get_triangle_mesh(0)])
+    rng = np.random.default_rng(7)
+    n = 512
+    q = np.zeros((n, 15), np.float32)
+    q[:, 0] = _lib.SHAPE_SPHERE
+    q[:, 1] = rng.uniform(0.05, 1.5, n)
+    q[:, 5:8] = np.stack([rng.uniform(-9, 9, n) + offset, rng.uniform(4, 9, n), rng.uniform(-9, 9, n) - offset], 1)
+    q[:, 11] = 1.0
+    q[:, 12:15] = np.stack([rng.uniform(-12, 12, n), rng.uniform(-14, -3, n), rng.uniform(-12, 12, n)], 1)
+    c = np.zeros(n, _lib.SHAPE_CAST_DTYPE)
+    c["shape_type"] = _lib.SHAPE_SPHERE
+    c["shape_params"], c["position"], c["quaternion"], c["displacement"] = q[:, 1:5], q[:, 5:8], q[:, 8:12], q[:, 12:15]
+    h = g.cast_shapes(c)
+    out, bo = o.cast_shapes(q.astype(np.float64))
+    hit = (h["body"] == 0) & (bo == 0)
+    assert (bo == 0).sum() > 300 and ((h["body"] == 0) == (bo == 0)).mean() >= 0.99
+    err = np.abs(h["fraction"][hit] - out[hit, 0]) * np.linalg.norm(q[hit, 12:15], axis=1)
+    assert np.quantile(err, 0.99) < 2e-3 + 10 * np.spacing(np.float32(offset)) and err.max() < 0.1
+
+
+@pytest.mark.parametrize("worlds,per", [(341, 3), (256, 4), (205, 5), (11, 93), (2, 512)])  # 1,023 to 1,025 bodies
+def test_queries_of_many_worlds_at_the_small_tree_sizes(gpu_lib, worlds, per):
+    """Every world holds the same row of spheres; a ray along a world's row, a cast and a point meet
+    that world's bodies only."""
+    n = worlds * per
+    b = scenes.blank_bodies(n)
+    k = np.arange(n)
+    scenes.set_sphere(b, k, 0.4)
+    b["position"][:, 0] = 2.0 + 2.0 * (k % per)
+    b["world"] = k // per
+    b["motion_type"] = _lib.STATIC
+    b["object_layer"] = scenes.LAYER_NOT_MOVING
+    g = make(scenes.Scene("rows", b, dt=1.0 / 60.0, steps=1, num_worlds=worlds))
+    w = np.arange(worlds)
+    rays = np.zeros((worlds, 8))
+    rays[:, 3], rays[:, 6], rays[:, 7] = 1.0, 4.0 * per, w
+    h = g.cast_rays(rays)
+    np.testing.assert_array_equal(h["body"], w * per)
+    np.testing.assert_allclose(h["fraction"] * rays[:, 6], 1.6, atol=2e-3)
+    c = np.zeros(worlds, _lib.SHAPE_CAST_DTYPE)
+    c["shape_type"], c["shape_params"][:, 0], c["quaternion"][:, 3], c["world"] = _lib.SHAPE_SPHERE, 0.1, 1.0, w
+    c["position"][:, 0], c["displacement"][:, 0] = 2.0 * per + 4.0, -4.0 * per  # from the row's far end
+    np.testing.assert_array_equal(g.cast_shapes(c)["body"], w * per + per - 1)
+    p = np.zeros(worlds, _lib.POINT_DTYPE)
+    p["position"][:, 0], p["world"] = 2.0 * per, w
+    inside = g.collide_points(p)
+    np.testing.assert_array_equal(inside["body"], w * per + per - 1)
+    assert (inside["count"] == 1).all()
