@@ -11,9 +11,12 @@
 // that share no body, other islands in the warp and later sweeps run side by side.
 // 18 islands of a 32-body world: 250 -> 110 us; 4,489 islands of 7,470 bodies: 464 us (per-thread)
 // beside 290 us (per-warp) -> 170 us.
-// One contact per lane costs a warp more instructions per contact than one island per thread
-// does when islands are chains, so from LANE_ISLANDS islands on, when the SMs are full either way,
-// the per-thread and per-warp classes keep them (325,318 islands: 1.2 ms + 0.5 ms).
+// One contact per lane costs a warp more instructions per contact than one island per thread does, so
+// above LANE_ISLANDS islands, when the SMs are full either way, the per-thread and per-warp classes
+// keep them: a step of 4,096 uneven worlds (325,297 islands) takes 6.45 ms on lanes and 6.08 ms so.
+// Below the line lanes win for every kind of island measured (steps of 8,000 alike: 5 contacts 0.82 and
+// 1.00 ms, 12 contacts 1.74 and 2.22, 22 contacts 3.35 and 3.71), and for islands that are all alike
+// also somewhat above it (32,000 of 5 contacts 1.83 and 2.29 ms, 64,000 3.12 and 3.20).
 #pragma once
 
 constexpr int LANE_ISLANDS = 16384;
@@ -41,11 +44,13 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_solve_lanes(DevWorld w, CacheTab
     CacheRecord *crecs = ct.recs[*ct.parity];
     // Islands by size, most contacts first: bucket rank 0 is the per-warp class's second bucket
     // (17-32 contacts), 1 its first (9-16), 2 + r the per-thread class's bucket SMALL_BUCKETS - 1 - r.
-    // A warp takes one island of the first two, 32 / k islands of k contacts of the others.
+    // A warp takes one island of the first, two of the second, 32 / k islands of k contacts of the others.
+    // (With one of the second as well, half the lanes had no contact: 8,000 islands of 12 contacts took
+    // 1,821 us, 1,436 on the per-warp class; two to a warp 930 us.)
     const int rank = min(lane, LANE_BUCKETS - 1);
     const int small_k = SMALL_BUCKETS + 1 - rank;
     const int have = rank < 2 ? w.ctr->mid_bucket[1 - rank] : w.ctr->small_bucket[small_k];
-    const int per = rank < 2 ? 1 : 32 / max(small_k, 1);
+    const int per = rank < 2 ? 1 + rank : 32 / max(small_k, 1);
     int items = lane < LANE_BUCKETS ? (have + per - 1) / per : 0;
     for (int o = 1; o < 32; o <<= 1) {  // inclusive scan: the buckets' ends
         const int v = __shfl_up_sync(FULL, items, o);
@@ -57,7 +62,7 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_solve_lanes(DevWorld w, CacheTab
         const int r = __popc(__ballot_sync(FULL, items <= item));  // the item's bucket
         const int first = r > 0 ? __shfl_sync(FULL, items, r - 1) : 0;
         const int count = __shfl_sync(FULL, have, r), group = __shfl_sync(FULL, per, r);
-        const int k = r < 2 ? 32 : SMALL_BUCKETS + 1 - r;  // lanes per island (0: islands without contacts)
+        const int k = r < 2 ? 32 >> r : SMALL_BUCKETS + 1 - r;  // lanes per island (0: islands without contacts)
         const int *list = r < 2 ? w.mid_list + (size_t)(1 - r) * w.cap : small_list + (size_t)k * w.cap;
         const int i0 = (item - first) * group, ni = min(group, count - i0);
         // ---- this lane's island and contact ----
@@ -73,7 +78,7 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_solve_lanes(DevWorld w, CacheTab
             island_iterations(w, isl, c_settings.vel_iters, c_settings.pos_iters, vel_iters, pos_iters);
         }
         const bool has = k > 0 && in_group && c_in < nc;
-        const int slots = r < 2 ? 64 : k + 1;  // body slots per island: k contacts join at most k + 1 bodies
+        const int slots = r < 2 ? 64 >> r : k + 1;  // body slots per island: k contacts join at most k + 1 bodies
         const bool vel = phase != SOLVE_POSITION;
         // ---- bodies ----
         for (int i = lane; i < 64; i += 32) {

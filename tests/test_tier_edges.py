@@ -476,3 +476,23 @@ def test_queries_of_many_worlds_at_the_small_tree_sizes(gpu_lib, worlds, per):
     inside = g.collide_points(p)
     np.testing.assert_array_equal(inside["body"], w * per + per - 1)
     assert (inside["count"] == 1).all()
+
+
+@pytest.mark.parametrize("worlds", [1, 2, 3, 7])
+@pytest.mark.parametrize("scene", [("pyramid", 3), ("stack", 9), ("stack", 16), ("pyramid", 4)])  # 12, 9, 16, 22 contacts
+def test_lane_islands_that_share_a_warp(gpu_lib, scene, worlds, monkeypatch):
+    """Islands of 9 to 16 contacts go two to a warp, the last one alone; against one thread each."""
+    kind, size = scene
+    sc = scenes.box_pyramid(size) if kind == "pyramid" else scenes.box_stack(height=size)
+    b = np.tile(sc.bodies, worlds)
+    b["world"] = np.repeat(np.arange(worlds), sc.n)
+    b["linear_velocity"][b["motion_type"] == 2] += np.random.default_rng(worlds).normal(
+        scale=0.1, size=((b["motion_type"] == 2).sum(), 3))  # no two islands alike
+    sc = scenes.Scene("tiled", b, dt=1.0 / 60.0, steps=1, num_worlds=worlds)
+    g = make(sc)
+    monkeypatch.setenv("CRASHCAT_SMALL_ISLAND_MAX", "64")
+    ref = make(sc)
+    for _ in range(3):
+        g.step(sc.dt, 1)
+        ref.step(sc.dt, 1)
+    np.testing.assert_allclose(g.get_state()[0], ref.get_state()[0], atol=1e-6)
