@@ -2299,10 +2299,6 @@ __device__ void epa_finish(const DevWorld &w, EpaItem &it, bool ok, R maxSep, V<
     it.pad = __float_as_int((float)(penetration));
 }
 
-// Packed pass.  fetch_warp = 1: the lanes of a warp run their items in lock-step rounds
-// (epa_round), a warp's worth of items after another; fetch_warp = 0: each thread takes its
-// next item as soon as it finishes one and runs it alone (epa).  Items that outgrow the packed
-// limits go to the fallback list.
 // one item's supports: a mesh triangle's (T: the world has triangle meshes) or a convex pair's
 template <bool H, bool T>
 __device__ __forceinline__ void epa_supports(const DevWorld &w, const EpaItem &it, Sup<R, H> &A, Sup<R, H, T> &B,
@@ -2333,6 +2329,10 @@ __device__ __forceinline__ void epa_packed_item(DevWorld &w, EpaItem *items, int
     epa_finish(w, it, ok, maxSep, axis, pa, pb);
 }
 
+// Packed pass.  fetch_warp = 1: the lanes of a warp run their items in lock-step rounds
+// (epa_round), a warp's worth of items after another; fetch_warp = 0: each thread takes its
+// next item as soon as it finishes one and runs it alone (epa).  Items that outgrow the packed
+// limits go to the fallback list.
 // H: the world has convex hulls (without them the support code leaves the hull loop out); T: it has
 // triangle meshes.  A mesh triangle's items run here too: a pass of their own on 1,024 threads took
 // 9.0 of the 24.5 ms of a step of 6,000 bodies on a terrain mesh (16 of the 152 SMs at work).
@@ -3441,8 +3441,9 @@ __device__ void ccd_cast_mesh(const DevWorld &w, uint32_t fa, float4 sa, float3 
         // hit hold no hit and are skipped; the rest are visited in the same order.  reach is the
         // radius and the error of the tests below: their squared distances carry rounding errors of
         // about 2^-24 of the squared lengths they subtract, bounded here with a factor of 64 to
-        // spare.  Where a length is not a number no node is skipped.  The mesh pass of 16,384 sweeps of 40-100 m over a 160 x 160-cell
-        // terrain: 20.5 -> 1.24 ms (a sphere's sweep had tested thousands of triangles).
+        // spare.  Where a length is not a number no node is skipped.  The mesh pass of
+        // 16,384 sweeps of 40-100 m over a 160 x 160-cell terrain: 20.5 -> 2.3 ms (a sphere's sweep had
+        // tested thousands of triangles).
         const float len = sqrtf(lensq3(dInB));
         const float3 rdir = len > 1e-10f ? dInB * (1.f / len) : f3(0.f, 0.f, 0.f);
         const float far = len + sqrtf(lensq3(f3(fmaxf(fabsf(start.x), fabsf(end.x)), fmaxf(fabsf(start.y), fabsf(end.y)),
